@@ -12,10 +12,12 @@
 // The scale searches compare sums of f32 products whose rounding decides which candidate wins, so the arithmetic is
 // the reference's operation for operation: this file is compiled with -fmad=false (no multiply-add contraction, as the
 // reference's LlamaCpp mode, utils.rs:37-45), divisions and square roots are IEEE, and sums run in the same order.
-// One thread packs one block (32 values for Q8_0, a 256-value superblock otherwise): the searches are sequential per
-// sub-block, and a matrix has hundreds of thousands of blocks.
+// One thread searches one sub-block (32 values of Q4_K, 16 of Q6_K) held in registers; the lanes of a superblock then meet in
+// shuffles to agree on its scales and to write its bytes. The searches are bound by the f32 pipe, not by memory: a sub-block
+// of Q4_K tries 21 scales over 32 values, a dozen operations each, and every sum has one order to run in.
 #include "common.cuh"
 #include "runtime.h"
+#include <type_traits>
 
 namespace b200q {
 
@@ -41,30 +43,54 @@ __device__ __forceinline__ int sat_i8(float v) {
 // ---------------------------------------------------------------------------------------------
 // Q8_0: d = amax / 127, q = round_half_away(x * (1 / d))
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float* __restrict__ x, uint8_t* __restrict__ out, long long nblocks) {
-    const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nblocks) return;
-    const float* xb = x + b * 32;
-    float amax = 0.0f;
-    for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(xb[i]));
+// HBM-bound: 4 bytes in and 1.06 out per value. Eight lanes share a block (one 128-bit load each); the 32 blocks of a CTA
+// are 1088 bytes, a multiple of 16, so they are put together in shared memory and leave as 128-bit stores.
+constexpr int Q8_CTA_BLOCKS = 32;
+__global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float* __restrict__ x, uint8_t* __restrict__ out, long long nblocks, int vec_in,
+                                                           int vec_out) {
+    __shared__ __align__(16) uint8_t stage[Q8_CTA_BLOCKS * Q8_0_BYTES];
+    const int tid = threadIdx.x, sub = tid & 7, local = tid >> 3;
+    const long long b0 = (long long)blockIdx.x * Q8_CTA_BLOCKS, b = b0 + local;
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (b < nblocks) {
+        const float* xb = x + b * 32 + 4 * sub;
+        if (vec_in) {
+            const float4 t = __ldg(reinterpret_cast<const float4*>(xb));
+            v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = xb[i];
+        }
+    }
+    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+#pragma unroll
+    for (int m = 4; m > 0; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
     const float d = amax / 127.0f;
     const float id = d != 0.0f ? 1.0f / d : 0.0f;
-    // a block is 34 bytes at a 2-byte-aligned address: seventeen 16-bit stores
-    unsigned short* o = reinterpret_cast<unsigned short*>(out + b * Q8_0_BYTES);
-    o[0] = f16_bits(d);
-    for (int i = 0; i < 16; ++i) {
-        const unsigned lo = (unsigned)sat_i8(roundf(xb[2 * i] * id)) & 0xffu;
-        const unsigned hi = (unsigned)sat_i8(roundf(xb[2 * i + 1] * id)) & 0xffu;
-        o[1 + i] = (unsigned short)(lo | (hi << 8));
+    unsigned short* o = reinterpret_cast<unsigned short*>(stage + local * Q8_0_BYTES);
+    if (sub == 0) o[0] = f16_bits(d);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const unsigned lo = (unsigned)sat_i8(roundf(v[2 * i] * id)) & 0xffu;
+        const unsigned hi = (unsigned)sat_i8(roundf(v[2 * i + 1] * id)) & 0xffu;
+        o[1 + 2 * sub + i] = (unsigned short)(lo | (hi << 8));
     }
+    __syncthreads();
+    const int bytes = (int)min((long long)Q8_CTA_BLOCKS, nblocks - b0) * Q8_0_BYTES;
+    uint8_t* dst = out + b0 * Q8_0_BYTES;
+    const int whole = vec_out ? bytes / 16 : 0;
+    for (int i = tid; i < whole; i += 256) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(stage)[i];
+    for (int i = whole * 8 + tid; i < bytes / 2; i += 256)
+        reinterpret_cast<unsigned short*>(dst)[i] = reinterpret_cast<const unsigned short*>(stage)[i];
 }
 
 // ---------------------------------------------------------------------------------------------
 // Q4_K
 // ---------------------------------------------------------------------------------------------
 // make_qkx2_quants(n = 32, nmax = 15, rmin = -1, rdelta = 0.1, nstep = 20, squared error): the weighted least-squares
-// search for (scale, min) of one sub-block. Returns the scale; *the_min = -min.
-__device__ float search_scale_min_q4(const float* x, const float* weights, uint8_t* L, float* the_min) {
+// search for (scale, min) of one sub-block. Returns the scale; *the_min = -min. This plain form serves the sub-blocks whose
+// range is too near the ends of the f32 range for the bounds of the register form below, and those with a NaN or an infinity.
+__device__ __noinline__ float search_scale_min_q4(const float* x, const float* weights, uint8_t* L, float* the_min) {
     constexpr int n = 32, nmax = 15, nstep = 20;
     const float rmin = -1.0f, rdelta = 0.1f;
     float mn = x[0], mx = x[0];
@@ -140,71 +166,233 @@ __device__ __forceinline__ void scale_min_k4(int j, const uint8_t* q, int& sc, i
     }
 }
 
-__global__ void __launch_bounds__(64) quantize_q4_k_kernel(const float* __restrict__ xs, uint8_t* __restrict__ out, long long nblocks) {
-    const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nblocks) return;
-    const float* x = xs + b * QK_K;
-    uint8_t L[QK_K];
-    float mins[8], scales[8];
-    uint8_t packed_scales[12];
-    for (int i = 0; i < 12; ++i) packed_scales[i] = 0;
-    for (int j = 0; j < 8; ++j) {
-        float xv[32], weights[32];
-        float sumsq = 0.0f;
-        for (int i = 0; i < 32; ++i) {
-            xv[i] = x[32 * j + i];
-            sumsq = sumsq + xv[i] * xv[i];  // k_quants.rs:302-305
-        }
-        const float av_x = sqrtf(sumsq / 32.0f);
-        for (int i = 0; i < 32; ++i) weights[i] = av_x + fabsf(xv[i]);
-        scales[j] = search_scale_min_q4(xv, weights, L + 32 * j, &mins[j]);
+// clampi(nearest_int_mul(iscale, xm), 0, 15) as a float; HIGH: the product may be above 15
+template <bool HIGH> __device__ __forceinline__ float q4_level(float iscale, float xm) {
+    const float l = fmaxf(iscale * xm + ROUNDING_MAGIC, ROUNDING_MAGIC) - ROUNDING_MAGIC;
+    return HIGH ? fminf(l, 15.0f) : l;
+}
+// The same search with the sub-block in registers, levels as floats. The candidates depend on one another (a better one moves
+// the minimum that the next one's levels start from), so all 21 run, in the reference's order; about 18 f32 operations per value
+// and candidate are what this kernel is made of (14336 x 4096: 1262 us with a superblock per thread in local memory, 864 now; the
+// f32 pipe alone would need about 640). *bad: the range left the band in which a level's product is below 2^22 (then the
+// integer form above decides); *best_iscale, *best_mn: what the winning levels were made with.
+__device__ __forceinline__ float search_scale_min_q4_regs(const float (&x)[32], const float (&w)[32], float mn, float mx, float* the_min,
+                                                          float* best_iscale, float* best_mn, bool* bad) {
+    float best_error = 0.0f, sum_w = 0.0f, sum_x = 0.0f;
+    float iscale = 15.0f / (mx - mn);
+    float scale = 1.0f / iscale;
+    *best_iscale = iscale;
+    *best_mn = mn;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        sum_w = i == 0 ? w[0] : sum_w + w[i];
+        sum_x = i == 0 ? w[0] * x[0] : w[i] * x[i] + sum_x;
+        float diff = (scale * q4_level<true>(iscale, x[i] - mn) + mn) - x[i];
+        diff = diff * diff;
+        best_error = w[i] * diff + best_error;
     }
-    float max_scale = 0.0f, max_min = 0.0f;
-    for (int j = 0; j < 8; ++j) {
-        max_scale = fmaxf(scales[j], max_scale);
-        max_min = fmaxf(mins[j], max_min);
+    auto candidate = [&](auto clamp_high, int is) {
+        const float range = mx - mn;
+        if (!(range > 1e-36f)) *bad = true;
+        iscale = ((0.1f * (float)is + -1.0f) + 15.0f) / range;
+        float l[32];
+        float sum_l = 0.0f, sum_l2 = 0.0f, sum_xl = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            l[i] = q4_level<decltype(clamp_high)::value>(iscale, x[i] - mn);
+            const float wl = w[i] * l[i];
+            sum_l += wl;
+            sum_l2 = wl * l[i] + sum_l2;
+            sum_xl = wl * x[i] + sum_xl;
+        }
+        const float d = sum_w * sum_l2 - sum_l * sum_l;
+        float this_scale = -(sum_x * sum_l - sum_w * sum_xl) / d;
+        float this_min = (sum_l2 * sum_x - sum_l * sum_xl) / d;
+        if (this_min > 0.0f) {
+            this_min = 0.0f;
+            this_scale = sum_xl / sum_l2;
+        }
+        float err = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            float diff = (this_scale * l[i] + this_min) - x[i];
+            diff = diff * diff;
+            err = w[i] * diff + err;
+        }
+        if (d > 0.0f && err < best_error) {
+            best_error = err;
+            scale = this_scale;
+            *best_iscale = iscale;
+            *best_mn = mn;
+            mn = this_min;
+        }
+    };
+    // up to candidate 10 the largest product is 15 (1 + 2u), which rounds to 15 by itself
+#pragma unroll 1
+    for (int is = 0; is <= 10; ++is) candidate(std::false_type{}, is);
+#pragma unroll 1
+    for (int is = 11; is <= 20; ++is) candidate(std::true_type{}, is);
+    *the_min = -mn;
+    return scale;
+}
+
+// One lane per sub-block, eight lanes per superblock.
+constexpr int Q4_CTA_THREADS = 128;
+__global__ void __launch_bounds__(Q4_CTA_THREADS, 4) quantize_q4_k_kernel(const float* __restrict__ xs, uint8_t* __restrict__ out, long long nblocks,
+                                                                       int vec_in, int vec_out) {
+    __shared__ uint8_t slow_l[Q4_CTA_THREADS][32];  // levels of sub-blocks that took the plain search
+    const int tid = threadIdx.x, j = tid & 7;
+    const long long b_raw = ((long long)blockIdx.x * Q4_CTA_THREADS + tid) >> 3;
+    const bool valid = b_raw < nblocks;
+    const long long b = valid ? b_raw : nblocks - 1;  // (the lanes of a warp stay together: shuffles below)
+    const float* src = xs + b * QK_K + 32 * j;
+    float x[32], w[32];
+    float sumsq = 0.0f, mn, mx;
+    if (vec_in) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const float4 t = __ldg(reinterpret_cast<const float4*>(src) + i);
+            x[4 * i] = t.x; x[4 * i + 1] = t.y; x[4 * i + 2] = t.z; x[4 * i + 3] = t.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) x[i] = src[i];
+    }
+    mn = mx = x[0];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        sumsq = sumsq + x[i] * x[i];  // k_quants.rs:302-305
+        mn = fminf(mn, x[i]);
+        mx = fmaxf(mx, x[i]);
+    }
+    {
+        const float av_x = sqrtf(sumsq / 32.0f);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) w[i] = av_x + fabsf(x[i]);
+    }
+    if (mn > 0.0f) mn = 0.0f;
+    float scale, the_min, best_iscale, best_mn;
+    bool plain = !(sumsq < 1e35f);  // (false for a NaN as well)
+    if (mx == mn) {
+        scale = 0.0f;
+        the_min = -mn;
+        best_iscale = 0.0f;
+        best_mn = 0.0f;
+    } else {
+        scale = search_scale_min_q4_regs(x, w, mn, mx, &the_min, &best_iscale, &best_mn, &plain);
+        if (plain) {
+            float xv[32], wv[32];
+            for (int i = 0; i < 32; ++i) {
+                xv[i] = x[i];
+                wv[i] = w[i];
+            }
+            scale = search_scale_min_q4(xv, wv, slow_l[tid], &the_min);
+        }
+    }
+    float max_scale = fmaxf(scale, 0.0f), max_min = fmaxf(the_min, 0.0f);
+#pragma unroll
+    for (int m = 4; m > 0; m >>= 1) {
+        max_scale = fmaxf(max_scale, __shfl_xor_sync(0xffffffffu, max_scale, m));
+        max_min = fmaxf(max_min, __shfl_xor_sync(0xffffffffu, max_min, m));
     }
     const float inv_scale = max_scale > 0.0f ? 63.0f / max_scale : 0.0f;
     const float inv_min = max_min > 0.0f ? 63.0f / max_min : 0.0f;
-    for (int j = 0; j < 8; ++j) {
-        const int lsi = nearest_int_mul(inv_scale, scales[j]);
-        const int lmi = nearest_int_mul(inv_min, mins[j]);
-        const uint8_t ls = (uint8_t)(lsi < 63 ? lsi : 63);
-        const uint8_t lm = (uint8_t)(lmi < 63 ? lmi : 63);
-        if (j < 4) {
-            packed_scales[j] = ls;
-            packed_scales[j + 4] = lm;
-        } else {
-            packed_scales[j + 4] = (uint8_t)((ls & 0xF) | ((lm & 0xF) << 4));
-            packed_scales[j - 4] |= (uint8_t)((ls >> 4) << 6);
-            packed_scales[j] |= (uint8_t)((lm >> 4) << 6);
+    const int lsi = nearest_int_mul(inv_scale, scale);
+    const int lmi = nearest_int_mul(inv_min, the_min);
+    const unsigned ls = (uint8_t)(lsi < 63 ? lsi : 63), lm = (uint8_t)(lmi < 63 ? lmi : 63);
+    // every lane of the superblock builds the twelve bytes of packed 6-bit scales and mins (utils.rs:119-129 read backwards)
+    uint32_t sc_w = 0, m_w = 0, hi_w = 0;
+    {
+        const unsigned mine = ls | (lm << 8);
+        const int base = (tid & 31) & ~7;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const unsigned a = __shfl_sync(0xffffffffu, mine, base + q), c = __shfl_sync(0xffffffffu, mine, base + 4 + q);
+            const unsigned als = a & 0xffu, alm = a >> 8, cls = c & 0xffu, clm = c >> 8;
+            sc_w |= ((als | ((cls >> 4) << 6)) & 0xffu) << (8 * q);
+            m_w |= ((alm | ((clm >> 4) << 6)) & 0xffu) << (8 * q);
+            hi_w |= (((cls & 0xFu) | ((clm & 0xFu) << 4)) & 0xffu) << (8 * q);
         }
     }
     const unsigned short dh = f16_bits(max_scale / 63.0f), mh = f16_bits(max_min / 63.0f);
     const float dv = f16_value(dh), mv = f16_value(mh);
-    // every value again, against the scales as they are stored (k_quants.rs:1995-2005)
-    for (int j = 0; j < 8; ++j) {
-        int sc, m;
-        scale_min_k4(j, packed_scales, sc, m);
-        const float d = dv * (float)sc;
-        if (d != 0.0f) {
-            const float dm = mv * (float)m;
-            for (int ii = 0; ii < 32; ++ii) L[32 * j + ii] = (uint8_t)clampi(nearest_int((x[32 * j + ii] + dm) / d), 0, 15);
+    // the scale and min as they are stored, and every value again against them (k_quants.rs:1995-2005)
+    int sc, m;
+    {
+        const uint32_t words[3] = {sc_w, m_w, hi_w};
+        uint8_t packed[12];
+#pragma unroll
+        for (int i = 0; i < 12; ++i) packed[i] = (uint8_t)(words[i >> 2] >> (8 * (i & 3)));
+        // (both decodings, selected: j differs between the lanes)
+        int sc_lo = 0, m_lo = 0, sc_hi = 0, m_hi = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            int s0, m0, s1, m1;
+            scale_min_k4(q, packed, s0, m0);
+            scale_min_k4(q + 4, packed, s1, m1);
+            if ((j & 3) == q) {
+                sc_lo = s0; m_lo = m0; sc_hi = s1; m_hi = m1;
+            }
+        }
+        sc = j < 4 ? sc_lo : sc_hi;
+        m = j < 4 ? m_lo : m_hi;
+    }
+    const float d = dv * (float)sc, dm = mv * (float)m;
+    uint32_t lw[8];
+    if (d != 0.0f) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            lw[i] = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) lw[i] |= (uint32_t)clampi(nearest_int((x[4 * i + q] + dm) / d), 0, 15) << (8 * q);
+        }
+    } else {
+        // a sub-block whose stored scale is zero keeps the levels of its search
+        const bool from_plain = plain && mx != mn;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            lw[i] = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int e = 4 * i + q;
+                const uint32_t level = mx == mn ? 0u : (from_plain ? (uint32_t)slow_l[tid][e] : (uint32_t)(int)q4_level<true>(best_iscale, x[e] - best_mn));
+                lw[i] |= level << (8 * q);
+            }
         }
     }
+    // sub-blocks 2c and 2c + 1 share 32 bytes, low and high nibbles: each of the two lanes writes one half
+    uint32_t o4[4];
+    const bool odd = (j & 1) != 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? lw[i] : lw[4 + i], 1);
+        o4[i] = odd ? (got | (lw[4 + i] << 4)) : (lw[i] | (got << 4));
+    }
+    if (!valid) return;
     uint8_t* o = out + b * Q4_K_BYTES;
-    o[0] = (uint8_t)dh; o[1] = (uint8_t)(dh >> 8);
-    o[2] = (uint8_t)mh; o[3] = (uint8_t)(mh >> 8);
-    for (int i = 0; i < 12; ++i) o[4 + i] = packed_scales[i];
-    for (int c = 0; c < 4; ++c)
-        for (int l = 0; l < 32; ++l) o[16 + 32 * c + l] = (uint8_t)(L[64 * c + l] | (L[64 * c + 32 + l] << 4));
+    uint8_t* oq = o + 16 + 32 * (j >> 1) + (odd ? 16 : 0);
+    const uint32_t head[4] = {(uint32_t)dh | ((uint32_t)mh << 16), sc_w, m_w, hi_w};
+    if (vec_out) {
+        *reinterpret_cast<uint4*>(oq) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+        if (j == 0) *reinterpret_cast<uint4*>(o) = make_uint4(head[0], head[1], head[2], head[3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            reinterpret_cast<unsigned short*>(oq)[2 * i] = (unsigned short)o4[i];
+            reinterpret_cast<unsigned short*>(oq)[2 * i + 1] = (unsigned short)(o4[i] >> 16);
+            if (j == 0) {
+                reinterpret_cast<unsigned short*>(o)[2 * i] = (unsigned short)head[i];
+                reinterpret_cast<unsigned short*>(o)[2 * i + 1] = (unsigned short)(head[i] >> 16);
+            }
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
 // Q6_K
 // ---------------------------------------------------------------------------------------------
 // make_qx_quants(n = 16, nmax = 32, rmse_type = 1, no importance weights): weights x^2, 18 nudged candidates.
-__device__ float search_scale_q6(const float* x, int8_t* ls) {
+__device__ __noinline__ float search_scale_q6(const float* x, int8_t* ls) {
     constexpr int n = 16, nmax = 32;
     float mx = 0.0f, amax = 0.0f;
     for (int i = 0; i < n; ++i) {
@@ -248,53 +436,168 @@ __device__ float search_scale_q6(const float* x, int8_t* ls) {
     return scale;
 }
 
-__global__ void __launch_bounds__(64) quantize_q6_k_kernel(const float* __restrict__ xs, uint8_t* __restrict__ out, long long nblocks) {
-    const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nblocks) return;
-    const float* xb = xs + b * QK_K;
-    int8_t L[QK_K];
-    float scales[16];
-    float max_scale = 0.0f, max_abs_scale = 0.0f;
-    for (int ib = 0; ib < 16; ++ib) {
+// The same search on 16 values in registers, the levels as floats; *best_is: the candidate whose levels won (0: the first).
+// Every candidate has to run in the reference's order here: the test is against a running product, not an error.
+__device__ __forceinline__ float q6_candidate_iscale(int is, float mx) {
+    return is == 0 ? -32.0f / mx : -(0.1f * (float)is + 32.0f) / mx;
+}
+__device__ __forceinline__ float q6_level(float iscale, float x) {  // clampi(nearest_int_mul(iscale, x), -32, 31) as a float
+    return fminf(fmaxf((iscale * x + ROUNDING_MAGIC) - ROUNDING_MAGIC, -32.0f), 31.0f);
+}
+__device__ __forceinline__ float search_scale_q6_regs(const float (&x)[16], float mx, int* best_is) {
+    float w[16], wx[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        w[i] = x[i] * x[i];
+        wx[i] = w[i] * x[i];
+    }
+    float scale = 0.0f, best = 0.0f;
+    *best_is = 0;
+#pragma unroll 1
+    for (int it = 0; it < 19; ++it) {  // the first guess, then -9 .. -1, 1 .. 9
+        const int is = it == 0 ? 0 : (it <= 9 ? it - 10 : it - 9);
+        const float isc = q6_candidate_iscale(is, mx);
+        float sumlx = 0.0f, suml2 = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float l = q6_level(isc, x[i]);
+            sumlx = wx[i] * l + sumlx;
+            suml2 = (w[i] * l) * l + suml2;
+        }
+        if (it == 0) {
+            scale = suml2 != 0.0f ? sumlx / suml2 : 0.0f;
+            best = scale * sumlx;
+        } else if (suml2 > 0.0f && sumlx * sumlx > best * suml2) {
+            *best_is = is;
+            scale = sumlx / suml2;
+            best = scale * sumlx;
+        }
+    }
+    return scale;
+}
+
+// One lane per 16 values, sixteen lanes per superblock.
+constexpr int Q6_CTA_THREADS = 128;
+__global__ void __launch_bounds__(Q6_CTA_THREADS) quantize_q6_k_kernel(const float* __restrict__ xs, uint8_t* __restrict__ out, long long nblocks,
+                                                                       int vec_in) {
+    __shared__ int8_t slow_l[Q6_CTA_THREADS][16];  // levels of groups that took the plain search
+    const int tid = threadIdx.x, ib = tid & 15;
+    const long long b_raw = ((long long)blockIdx.x * Q6_CTA_THREADS + tid) >> 4;
+    const bool valid = b_raw < nblocks;
+    const long long b = valid ? b_raw : nblocks - 1;  // (the lanes of a warp stay together: shuffles below)
+    const float* src = xs + b * QK_K + 16 * ib;
+    float x[16];
+    if (vec_in) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 t = __ldg(reinterpret_cast<const float4*>(src) + i);
+            x[4 * i] = t.x; x[4 * i + 1] = t.y; x[4 * i + 2] = t.z; x[4 * i + 3] = t.w;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = src[i];
+    }
+    float mx = 0.0f, amax = 0.0f, zero = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float a = fabsf(x[i]);
+        if (a > amax) {
+            amax = a;
+            mx = x[i];
+        }
+        zero += x[i] * 0.0f;  // NaN where a value is infinite or NaN
+    }
+    float scale;
+    int best_is = 0;
+    bool from_plain = false;
+    const bool none = amax < GROUP_MAX_EPS;
+    if (zero == 0.0f) {
+        scale = none ? 0.0f : search_scale_q6_regs(x, mx, &best_is);
+    } else {
         float xv[16];
-        for (int i = 0; i < 16; ++i) xv[i] = xb[16 * ib + i];
-        const float scale = search_scale_q6(xv, L + 16 * ib);
-        scales[ib] = scale;
-        if (fabsf(scale) > max_abs_scale) {
-            max_abs_scale = fabsf(scale);
-            max_scale = scale;
+        for (int i = 0; i < 16; ++i) xv[i] = x[i];
+        scale = search_scale_q6(xv, slow_l[tid]);
+        from_plain = true;
+    }
+    // the scale of largest magnitude, the first of equals (the reference walks the groups in order)
+    float max_abs = fabsf(scale) > 0.0f ? fabsf(scale) : 0.0f, max_scale = max_abs > 0.0f ? scale : 0.0f;
+    int who = ib;
+#pragma unroll
+    for (int m = 8; m > 0; m >>= 1) {
+        const float oa = __shfl_xor_sync(0xffffffffu, max_abs, m), os = __shfl_xor_sync(0xffffffffu, max_scale, m);
+        const int ow = __shfl_xor_sync(0xffffffffu, who, m);
+        if (oa > max_abs || (oa == max_abs && ow < who)) {
+            max_abs = oa;
+            max_scale = os;
+            who = ow;
         }
     }
     // an all-zero superblock gives max_scale = 0, iscale = -inf, d = f16(-0.0), scales 0: as the reference
     const float iscale = -128.0f / max_scale;
     const unsigned short dh = f16_bits(1.0f / iscale);
     const float dv = f16_value(dh);
-    int8_t sc8[16];
-    for (int ib = 0; ib < 16; ++ib) {
-        // (-inf * 0 is a NaN whose mantissa bits differ between machines: the reference's host turns it into scale 0)
-        const int v = max_abs_scale == 0.0f ? 0 : nearest_int_mul(iscale, scales[ib]);
-        sc8[ib] = (int8_t)(v < 127 ? v : 127);
-    }
-    for (int j = 0; j < 16; ++j) {
-        const float d = dv * (float)sc8[j];
-        if (d == 0.0f) continue;
-        for (int ii = 0; ii < 16; ++ii) L[16 * j + ii] = (int8_t)(clampi(nearest_int(xb[16 * j + ii] / d), -32, 31) + 32);
-    }
-    uint8_t* o = out + b * Q6_K_BYTES;
-    for (int h = 0; h < 2; ++h) {
-        uint8_t* ql = o + 64 * h;
-        uint8_t* qh = o + 128 + 32 * h;
-        const int8_t* l = L + 128 * h;
-        for (int i = 0; i < 32; ++i) {
-            const int q1 = l[i], q2 = l[i + 32], q3 = l[i + 64], q4 = l[i + 96];
-            ql[i] = (uint8_t)((q1 & 0xF) | ((q3 & 0xF) << 4));
-            ql[i + 32] = (uint8_t)((q2 & 0xF) | ((q4 & 0xF) << 4));
-            qh[i] = (uint8_t)((q1 >> 4) | ((q2 >> 4) << 2) | ((q3 >> 4) << 4) | ((q4 >> 4) << 6));
+    // (-inf * 0 is a NaN whose mantissa bits differ between machines: the reference's host turns it into scale 0)
+    const int sv = max_abs == 0.0f ? 0 : nearest_int_mul(iscale, scale);
+    const int8_t sc8 = (int8_t)(sv < 127 ? sv : 127);
+    const float d = dv * (float)sc8;
+    uint32_t lw[4];  // sixteen 6-bit levels, four to a word
+    if (d != 0.0f) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            lw[i] = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) lw[i] |= (uint32_t)(clampi(nearest_int(x[4 * i + q] / d), -32, 31) + 32) << (8 * q);
+        }
+    } else {
+        // a group whose stored scale is zero keeps the levels of its search
+        const float isc = q6_candidate_iscale(best_is, mx);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            lw[i] = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int e = 4 * i + q;
+                const uint32_t level = from_plain ? (uint32_t)(uint8_t)slow_l[tid][e] : (none ? 0u : (uint32_t)((int)q6_level(isc, x[e]) + 32));
+                lw[i] |= (level & 0xffu) << (8 * q);
+            }
         }
     }
-    for (int ib = 0; ib < 16; ++ib) o[192 + ib] = (uint8_t)sc8[ib];
-    o[208] = (uint8_t)dh;
-    o[209] = (uint8_t)(dh >> 8);
+    // group ib is half h = ib >> 3, quarter qd, 16-value part g of it. ql byte (qd & 1, g, i) = low nibbles of quarters qd and
+    // qd ^ 2, qh byte (g, i) = the high two bits of all four quarters: lanes 4 and 2, 4 apart exchange
+    const int qd = (ib >> 1) & 3, g = ib & 1, h = ib >> 3;
+    uint32_t ql[2], qh = 0;
+    {
+        uint32_t lo[4], hi[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            lo[i] = lw[i] & 0x0f0f0f0fu;
+            hi[i] = ((lw[i] >> 4) & 0x03030303u) << (2 * qd);
+        }
+        const bool upper = qd >= 2;  // writes the second eight bytes of the sixteen that the two lanes share
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? lo[i] : lo[2 + i], 4);
+            ql[i] = upper ? (got | (lo[2 + i] << 4)) : (lo[i] | (got << 4));
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t t = hi[i] | __shfl_xor_sync(0xffffffffu, hi[i], 2);
+            t |= __shfl_xor_sync(0xffffffffu, t, 4);
+            if (i == qd) qh = t;  // lane qd writes word qd
+        }
+    }
+    if (!valid) return;
+    uint8_t* o = out + b * Q6_K_BYTES;  // 2-byte aligned
+    unsigned short* oql = reinterpret_cast<unsigned short*>(o + 64 * h + 32 * (qd & 1) + 16 * g + (qd >= 2 ? 8 : 0));
+    unsigned short* oqh = reinterpret_cast<unsigned short*>(o + 128 + 32 * h + 16 * g + 4 * qd);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        oql[2 * i] = (unsigned short)ql[i];
+        oql[2 * i + 1] = (unsigned short)(ql[i] >> 16);
+        oqh[i] = (unsigned short)(qh >> (16 * i));
+    }
+    o[192 + ib] = (uint8_t)sc8;
+    if (ib == 0) *reinterpret_cast<unsigned short*>(o + 208) = dh;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -355,9 +658,12 @@ int quantize_weights(int type, const float* x, void* out, long long n, cudaStrea
     if (n < 0 || n % type_block_elems(type) != 0 || reinterpret_cast<uintptr_t>(out) % 2 != 0) return B200Q_ERR_INVALID;
     if (n == 0) return 0;
     const long long nb = n / type_block_elems(type);
-    if (type == TYPE_Q8_0) quantize_q8_0_kernel<<<(unsigned)((nb + 255) / 256), 256, 0, s>>>(x, static_cast<uint8_t*>(out), nb);
-    else if (type == TYPE_Q4_K) quantize_q4_k_kernel<<<(unsigned)((nb + 63) / 64), 64, 0, s>>>(x, static_cast<uint8_t*>(out), nb);
-    else quantize_q6_k_kernel<<<(unsigned)((nb + 63) / 64), 64, 0, s>>>(x, static_cast<uint8_t*>(out), nb);
+    const int vec_in = reinterpret_cast<uintptr_t>(x) % 16 == 0, vec_out = reinterpret_cast<uintptr_t>(out) % 16 == 0;
+    uint8_t* o = static_cast<uint8_t*>(out);
+    const auto ctas = [](long long items, int per_cta) { return (unsigned)((items + per_cta - 1) / per_cta); };
+    if (type == TYPE_Q8_0) quantize_q8_0_kernel<<<ctas(nb, Q8_CTA_BLOCKS), 256, 0, s>>>(x, o, nb, vec_in, vec_out);
+    else if (type == TYPE_Q4_K) quantize_q4_k_kernel<<<ctas(8 * nb, Q4_CTA_THREADS), Q4_CTA_THREADS, 0, s>>>(x, o, nb, vec_in, vec_out);
+    else quantize_q6_k_kernel<<<ctas(16 * nb, Q6_CTA_THREADS), Q6_CTA_THREADS, 0, s>>>(x, o, nb, vec_in);
     return (int)cudaGetLastError();
 }
 

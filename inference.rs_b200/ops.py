@@ -58,7 +58,8 @@ def quantize_weights(x: torch.Tensor, dtype: GgmlDType) -> torch.Tensor:
     n, k = x.shape
     nbytes = n * dtype.row_bytes(k)
     padding = MATRIX_ROW_PADDING * dtype.type_size // dtype.block_size
-    buf = torch.zeros(nbytes + padding, dtype=torch.uint8, device=x.device)
+    buf = torch.empty(nbytes + padding, dtype=torch.uint8, device=x.device)
+    buf[nbytes:].zero_()  # the quantizer writes every byte of the blocks
     kl.check(kl.library().b200q_quantize(int(dtype), x.data_ptr(), buf.data_ptr(), n * k, _stream()), "b200q_quantize")
     return buf
 

@@ -104,3 +104,37 @@ def test_quantize_errors_and_bad_row_ids():
     st = kl.device_status()
     assert st[0] == 6 and st[2] == 1, st  # code 6: row id outside the table; detail = position of the id
     kl.check(kl.library().b200q_reset_device_status(), "reset")
+
+
+def search_rows(k):
+    """Distributions that crowd the candidates of the scale searches together, or whose products leave the normal f32 range (above
+    1e6 the block scale itself no longer fits f16)."""
+    rng = np.random.default_rng(5)
+    g = rng.standard_normal((8, k))
+    return np.concatenate([g * s for s in (1e-36, 1e-30, 1e-18, 1e-12, 1e-6, 1.0, 1e4)] +
+                          [rng.standard_t(1.5, (16, k)), rng.uniform(0, 1, (8, k)), 1.0 + g * 1e-6, -3.0 + g * 1e-3, np.round(g * 2), np.sign(g),
+                           g * (rng.random((8, k)) < 0.05), np.repeat(g[:, ::32], 32, axis=1)]).astype(np.float32)
+
+
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("case", ["search", "tail", "unaligned"])
+def test_register_searches_pick_the_oracles_candidate(type_id, case):
+    """Levels kept as floats, and the sub-blocks that fall back to the integer form (search); block counts that fill neither a CTA
+    nor a warp (tail); an input on a 4-byte and an output on a 2-byte boundary (unaligned)."""
+    from inference_rs_b200 import kernel_library as kl
+    if case == "search":
+        w = search_rows(1024)
+    else:
+        w = seeded_weights(7 if case == "tail" else 33, 256, 21)
+    n, k = w.shape
+    want = kq.quantize(type_id, w).reshape(-1)
+    shift = 2 if case == "unaligned" else 0
+    src = torch.zeros(n * k + 4, device="cuda")
+    x = src[1:1 + n * k] if case == "unaligned" else src[:n * k]
+    x.copy_(torch.from_numpy(w.reshape(-1)))
+    out = torch.zeros(want.size + shift + 16, dtype=torch.uint8, device="cuda")
+    kl.check(kl.library().b200q_quantize(int(DT[type_id]), x.data_ptr(), out.data_ptr() + shift, n * k, torch.cuda.current_stream().cuda_stream))
+    torch.cuda.synchronize()
+    got = out.cpu().numpy()
+    assert np.array_equal(got[shift:shift + want.size], want)
+    assert not got[:shift].any() and not got[shift + want.size:].any(), "bytes outside the blocks were written"
