@@ -138,3 +138,22 @@ def test_register_searches_pick_the_oracles_candidate(type_id, case):
     got = out.cpu().numpy()
     assert np.array_equal(got[shift:shift + want.size], want)
     assert not got[:shift].any() and not got[shift + want.size:].any(), "bytes outside the blocks were written"
+
+
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("n,k", [(1, 256), (3, 2816), (129, 256)])
+def test_dequantize_rows_of_any_width_and_alignment(type_id, n, k):
+    from inference_rs_b200 import kernel_library as kl
+    packed = kq.quantize(type_id, seeded_weights(n, k, 15))
+    want = kq.dequantize(type_id, packed, k)
+    flat = packed.reshape(-1)
+    for w_off, o_off in ((0, 0), (2, 0), (1, 0), (0, 4)):
+        buf = torch.zeros(flat.size + 64, dtype=torch.uint8, device="cuda")
+        buf[w_off:w_off + flat.size].copy_(torch.from_numpy(flat.copy()))
+        out = torch.zeros(n * k + 8, device="cuda")
+        kl.check(kl.library().b200q_dequantize(int(DT[type_id]), 0, buf.data_ptr() + w_off, out.data_ptr() + o_off, n, k,
+                                               torch.cuda.current_stream().cuda_stream))
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        assert np.array_equal(got[o_off // 4:o_off // 4 + n * k].reshape(n, k), want)
+        assert not got[:o_off // 4].any() and not got[o_off // 4 + n * k:].any()
