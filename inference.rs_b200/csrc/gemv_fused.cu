@@ -55,7 +55,7 @@ struct GemvGluParams {
 
 // One CTA per SM, 16 consumer warps + 1 producer warp, as gemv_staged_kernel; NREG = register-resident item slots.
 template <int TYPE, int B, typename dst_t, int NREG>
-__global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_glu_kernel(const GemvGluParams p) {
+__global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_glu_kernel(GemvGluParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);
     uint64_t* empty = full + GEMV_MAX_STAGES;
@@ -326,6 +326,14 @@ __global__ void __launch_bounds__(256) gemv_glu_simple_kernel(const uint8_t* __r
     }
 }
 
+template <void (*kernel)(GemvGluParams)>
+static int launch_glu_kernel(int grid, size_t smem, const GemvGluParams& p, cudaStream_t s) {
+    const cudaError_t e = allow_full_smem<kernel>();
+    if (e != cudaSuccess) return (int)e;
+    kernel<<<grid, GEMV_THREADS, smem, s>>>(p);
+    return (int)cudaGetLastError();
+}
+
 template <int TYPE, int B, typename dst_t>
 static int launch_glu_b(const void* wg, const void* wu, const void* vy, void* dst, int K, int N, int stride_act, int stride_dst,
                         int activation, cudaStream_t s) {
@@ -335,23 +343,32 @@ static int launch_glu_b(const void* wg, const void* wu, const void* vy, void* ds
     GemvGluParams p{};
     size_t smem = 0;
     if (ring_ok) {
+        // A stage holds R rows of each matrix: whole passes of all warps, starting on 16-byte boundaries. (The plan's own
+        // row_align may be a whole single-matrix stage, its unit of partition between CTAs: two of those do not fit the ring
+        // twice, and Q4_K 4096 x 14336 fell through to the plain kernel below, 101 us instead of 13.)
         const int islots = 1 << one.p.log2_islots;
         const int rows_per_pass = (GEMV_CONSUMER_WARPS / one.p.warps_per_row) * (32 / islots);
-        const int unit = rows_per_pass * one.p.row_align / gcd_int(rows_per_pass, one.p.row_align);
+        const int align16 = 16 / gcd_int(one.p.row_bytes, 16);
+        const int unit = rows_per_pass * align16 / gcd_int(rows_per_pass, align16);
         int R = one.p.rows_per_stage / 2 / unit * unit;
         if (R < unit) R = unit;
-        p.rows_per_stage = R;
-        p.half_bytes = (R * one.p.row_bytes + 16 + 15) & ~15;
-        p.stage_bytes = (2 * p.half_bytes + 127) & ~127;
         const int budget = runtime_info().smem_optin - 1024;
         const int wpr = one.p.warps_per_row;
         int S;
-        for (S = GEMV_MAX_STAGES; S >= 2; --S) {
-            const int combine = wpr > 1 ? (((S * R * wpr * 2 * B + S * R) * 4 + 127) & ~127) : 0;
-            if (GEMV_BARRIER_BYTES + one.p.act_bytes + combine + S * p.stage_bytes <= budget) {
-                smem = (size_t)GEMV_BARRIER_BYTES + one.p.act_bytes + combine + (size_t)S * p.stage_bytes;
-                break;
+        for (;;) {
+            p.rows_per_stage = R;
+            p.half_bytes = (R * one.p.row_bytes + 16 + 15) & ~15;
+            p.stage_bytes = (2 * p.half_bytes + 127) & ~127;
+            for (S = GEMV_MAX_STAGES; S >= 2; --S) {
+                const int combine = wpr > 1 ? (((S * R * wpr * 2 * B + S * R) * 4 + 127) & ~127) : 0;
+                if (GEMV_BARRIER_BYTES + one.p.act_bytes + combine + S * p.stage_bytes <= budget) {
+                    smem = (size_t)GEMV_BARRIER_BYTES + one.p.act_bytes + combine + (size_t)S * p.stage_bytes;
+                    break;
+                }
             }
+            // several rows of activations leave less room: then fewer rows than a pass, as the single-matrix plan
+            if (S >= 2 || R <= align16 || (R / 2) % align16 != 0) break;
+            R /= 2;
         }
         ring_ok = S >= 2;
         p.nstages = S;
@@ -380,15 +397,11 @@ static int launch_glu_b(const void* wg, const void* wu, const void* vy, void* ds
     p.act_bytes = one.p.act_bytes;
     p.activation = activation;
     p.status = status_ptr();
-    auto launch = [&](auto kernel) -> int {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, runtime_info().smem_optin - 1024);
-        if (e != cudaSuccess) return (int)e;
-        kernel<<<one.grid, GEMV_THREADS, smem, s>>>(p);
-        return (int)cudaGetLastError();
-    };
     // register-resident activations where the single-matrix plan has them (one or two rows of activations, one slot)
-    if (one.nreg == 1 && B <= 2) return launch(gemv_glu_kernel<TYPE, B, dst_t, (B <= 2 ? 1 : 0)>);
-    return launch(gemv_glu_kernel<TYPE, B, dst_t, 0>);
+    if constexpr (B <= 2) {
+        if (one.nreg == 1) return launch_glu_kernel<gemv_glu_kernel<TYPE, B, dst_t, 1>>(one.grid, smem, p, s);
+    }
+    return launch_glu_kernel<gemv_glu_kernel<TYPE, B, dst_t, 0>>(one.grid, smem, p, s);
 }
 
 template <int TYPE, typename dst_t>

@@ -1637,6 +1637,23 @@ static inline int launch_gemv(const void* vx, const void* act, void* dst, int K,
     }
 }
 
+template <auto kernel>
+static inline int launch_group_kernel(int grid, size_t smem, const GemvGroupParams& p, cudaStream_t s) {
+    const cudaError_t e = allow_full_smem<kernel>();
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid, 1, 1);
+    cfg.blockDim = dim3(GEMV_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.use_pdl ? 1 : 0;
+    return (int)cudaLaunchKernelEx(&cfg, kernel, p);
+}
+
 // Plans and launches a grouped GEMV (one activation row). Returns B200Q_ERR_UNSUPPORTED when the group does not fit
 // the staged kernel's preconditions; the caller then launches the matrices one by one.
 template <typename dst_t, int ACT = ACT_RAW_Q8_1>
@@ -1713,32 +1730,17 @@ static inline int launch_gemv_group(int nmat, const int* types, const void* cons
     smem += ar_bytes;
     if (exchange) p.px = *px;
     const int nreg = ipl <= 2 ? ipl : 0;
-    auto launch = [&](auto kernel) -> int {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rt.smem_optin - 1024);
-        if (e != cudaSuccess) return (int)e;
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3((unsigned)grid, 1, 1);
-        cfg.blockDim = dim3(GEMV_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = p.use_pdl ? 1 : 0;
-        return (int)cudaLaunchKernelEx(&cfg, kernel, p);
-    };
     using act_t = typename std::conditional<ACT == ACT_Q8_1, float, dst_t>::type;
     if constexpr (ACT == ACT_RAW_Q8_1) {
         if (exchange) {
-            if (nreg == 1) return launch(gemv_group_kernel<dst_t, act_t, 1, ACT, true>);
-            if (nreg == 2) return launch(gemv_group_kernel<dst_t, act_t, 2, ACT, true>);
-            return launch(gemv_group_kernel<dst_t, act_t, 0, ACT, true>);
+            if (nreg == 1) return launch_group_kernel<gemv_group_kernel<dst_t, act_t, 1, ACT, true>>(grid, smem, p, s);
+            if (nreg == 2) return launch_group_kernel<gemv_group_kernel<dst_t, act_t, 2, ACT, true>>(grid, smem, p, s);
+            return launch_group_kernel<gemv_group_kernel<dst_t, act_t, 0, ACT, true>>(grid, smem, p, s);
         }
     }
-    if (nreg == 1) return launch(gemv_group_kernel<dst_t, act_t, 1, ACT>);
-    if (nreg == 2) return launch(gemv_group_kernel<dst_t, act_t, 2, ACT>);
-    return launch(gemv_group_kernel<dst_t, act_t, 0, ACT>);
+    if (nreg == 1) return launch_group_kernel<gemv_group_kernel<dst_t, act_t, 1, ACT>>(grid, smem, p, s);
+    if (nreg == 2) return launch_group_kernel<gemv_group_kernel<dst_t, act_t, 2, ACT>>(grid, smem, p, s);
+    return launch_group_kernel<gemv_group_kernel<dst_t, act_t, 0, ACT>>(grid, smem, p, s);
 }
 
 // One weight type's dispatcher over the output element type; defined once per type in gemv_<type>.cu.

@@ -75,6 +75,13 @@ struct PerDeviceOnce {
     }
 };
 
+// All the dynamic shared memory a CTA may have, for one kernel (the template argument keeps the flags of kernels with the
+// same parameter type apart).
+template <auto kernel> cudaError_t allow_full_smem() {
+    static PerDeviceOnce configured;
+    return configured.run([] { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, runtime_info().smem_optin - 1024); });
+}
+
 int note_launch_status(int status);  // remembers the first non-zero status; returns its argument
 int take_launch_status();            // returns and clears it
 
