@@ -18,6 +18,8 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "lib", "sm100a")
 LIB = os.path.join(OUT_DIR, "libinferencequant_b200.so")
 OBJ_DIR = os.path.join(HERE, "build")
+HOST_SRC = os.path.join(CSRC, "host", "torch_host.cpp")
+HOST_LIB = os.path.join(HERE, "lib", "b200q_torch_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -69,8 +71,38 @@ def _compile(nvcc: str, src: str, obj: str, extra: list[str]) -> tuple[str, str]
     return src, res.stdout + res.stderr
 
 
+def build_host(force: bool = False, verbose: bool = False) -> str:
+    """The torch front end's native call path (a CPython extension against this interpreter's torch), if anything changed."""
+    import importlib.util
+    import sysconfig
+
+    torch_dir = next(iter(importlib.util.find_spec("torch").submodule_search_locations))
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DAT_PER_OPERATOR_HEADERS",
+           f"-I{torch_dir}/include", f"-I{torch_dir}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
+           f"-I{os.path.dirname(os.path.dirname(_nvcc()))}/include", HOST_SRC, f"-L{torch_dir}/lib",
+           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    h = hashlib.sha256(repr(cmd).encode() + sys.version.encode())
+    for path in (HOST_SRC, os.path.join(torch_dir, "version.py")):
+        with open(path, "rb") as fh:
+            h.update(fh.read())
+    digest_file = HOST_LIB + ".digest"
+    if not force and os.path.exists(HOST_LIB) and os.path.exists(digest_file) and open(digest_file).read() == h.hexdigest():
+        return HOST_LIB
+    os.makedirs(os.path.dirname(HOST_LIB), exist_ok=True)
+    res = subprocess.run([*cmd, "-o", HOST_LIB + ".tmp"], capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{res.stdout}\n{res.stderr}")
+    os.replace(HOST_LIB + ".tmp", HOST_LIB)
+    with open(digest_file, "w") as fh:
+        fh.write(h.hexdigest())
+    if verbose:
+        print(f"compiled {os.path.basename(HOST_SRC)}", file=sys.stderr)
+    return HOST_LIB
+
+
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
-    """Build the shared library if any source changed; return its path."""
+    """Build the shared library (and the torch front end's native part) if any source changed; return its path."""
+    build_host(force, verbose)
     hdr = _headers_digest()
     # one digest over every source: a library built from these exact sources is reused even where the object
     # directory did not travel with it

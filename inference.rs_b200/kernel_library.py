@@ -11,6 +11,7 @@ import os
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_NAME = "libinferencequant_b200.so"
+HOST_LIB_NAME = "b200q_torch_host.so"
 ARCH_DIR = "sm100a"
 
 
@@ -121,6 +122,36 @@ def library() -> C.CDLL:
             raise KernelLibraryError(f"{library_path()} lacks symbols: {missing}")
         _lib = lib
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The torch front end's native call path (csrc/host/torch_host.cpp), bound to `library()`; raises KernelLibraryError if it
+    was not built."""
+    global _host
+    if _host is None:
+        from importlib.machinery import ExtensionFileLoader
+        from importlib.util import module_from_spec, spec_from_file_location
+        path = os.path.join(HERE, "lib", HOST_LIB_NAME)
+        if not os.path.exists(path):
+            raise KernelLibraryError(f"{path} not found; build it with `python inference.rs_b200/build.py`.")
+        name = HOST_LIB_NAME.split(".")[0]
+        spec = spec_from_file_location(name, path, loader=ExtensionFileLoader(name, path))
+        mod = module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        lib = library()
+        mod.bind({sym: C.cast(getattr(lib, sym), _vp).value for sym in mod.symbols()}, check, launch_failed)
+        _host = mod
+    return _host
+
+
+def launch_failed(rc: int, what: str) -> None:
+    """A status that a void launcher left behind (`b200q_take_launch_status`)."""
+    err = KernelLibraryError(f"{what} failed with status {rc}")
+    err.status = rc
+    raise err
 
 
 def build_id() -> str:

@@ -1,10 +1,13 @@
 """torch-tensor front end of the C ABI: device memory and streams come from torch, the arithmetic from the library.
 
-Every function launches on torch's current CUDA stream and raises if the kernel library is unavailable.
+Every function launches on torch's current CUDA stream and raises if the kernel library is unavailable. The functions of the
+matmul path hand their arguments to the native call path (csrc/host/torch_host.cpp); what it does not take as it stands it
+declines with None, and the Python form below it raises the error or deals with the case.
 """
 from __future__ import annotations
 
 import ctypes as C
+import functools
 
 import numpy as np
 import torch
@@ -52,6 +55,9 @@ def upload_weights(packed: np.ndarray | torch.Tensor, dtype: GgmlDType, device="
 def quantize_weights(x: torch.Tensor, dtype: GgmlDType) -> torch.Tensor:
     """`b200q_quantize`: f32 [n, k] on the device -> packed blocks followed by the reference's padding (a buffer
     `upload_weights` would have produced), byte for byte the reference CPU quantizer's."""
+    buf = kl.host().quantize(dtype, x)
+    if buf is not None:
+        return buf
     _require_cuda(x)
     if x.dtype != torch.float32:
         raise TypeError("weights are quantized from f32")
@@ -66,6 +72,9 @@ def quantize_weights(x: torch.Tensor, dtype: GgmlDType) -> torch.Tensor:
 
 def dequantize(dtype: GgmlDType, w: torch.Tensor, n: int, k: int, out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
     """`b200q_dequantize`: packed [n, k] -> values [n, k] of `out_dtype`."""
+    out = kl.host().dequantize(dtype, w, n, k, elem_of(out_dtype))
+    if out is not None:
+        return out
     _require_cuda(w)
     out = torch.empty((n, k), dtype=out_dtype, device=w.device)
     kl.check(kl.library().b200q_dequantize(int(dtype), elem_of(out_dtype), w.data_ptr(), out.data_ptr(), n, k, _stream()), "b200q_dequantize")
@@ -74,19 +83,25 @@ def dequantize(dtype: GgmlDType, w: torch.Tensor, n: int, k: int, out_dtype: tor
 
 def get_rows(dtype: GgmlDType, w: torch.Tensor, ids: torch.Tensor, n: int, k: int, out_dtype: torch.dtype = torch.float32) -> torch.Tensor:
     """`b200q_get_rows`: rows `ids` (int32, any shape) of a packed [n, k] table -> [*ids.shape, k] of `out_dtype`."""
+    elem = elem_of(out_dtype)
+    out = kl.host().get_rows(dtype, w, ids, n, k, elem)
+    if out is not None:
+        return out
     _require_cuda(w)
-    flat = ids.reshape(-1).to(device=w.device, dtype=torch.int32).contiguous()
-    out = torch.empty((flat.numel(), k), dtype=out_dtype, device=w.device)
-    kl.check(kl.library().b200q_get_rows(int(dtype), elem_of(out_dtype), w.data_ptr(), flat.data_ptr(), out.data_ptr(), flat.numel(), k, n,
-                                         _stream()), "b200q_get_rows")
-    return out.reshape(*ids.shape, k)
+    out = kl.host().get_rows(dtype, w, ids.to(device=w.device, dtype=torch.int32).contiguous(), n, k, elem)
+    if out is None:
+        raise TypeError("get_rows takes packed weights and integer ids")
+    return out
 
 
 def quantize_q8_1(x: torch.Tensor, k_padded: int | None = None) -> torch.Tensor:
     """`launch_mmvq_gguf_quantize_q8_1_<dtype>`: x [rows, k] -> uint8 [rows, k_padded / 32 * 36]."""
+    k_padded = pad(x.shape[-1], MATRIX_ROW_PADDING) if k_padded is None else k_padded
+    out = kl.host().quantize_q8_1(x, k_padded)
+    if out is not None:
+        return out
     _require_cuda(x)
     rows, k = x.shape
-    k_padded = pad(k, MATRIX_ROW_PADDING) if k_padded is None else k_padded
     out = torch.empty((rows, k_padded // 32 * 36), dtype=torch.uint8, device=x.device)
     fn = getattr(kl.library(), f"launch_mmvq_gguf_quantize_q8_1_{ELEM_TAG[elem_of(x.dtype)]}")
     fn(x.data_ptr(), out.data_ptr(), k, k_padded, rows, _stream())
@@ -95,9 +110,12 @@ def quantize_q8_1(x: torch.Tensor, k_padded: int | None = None) -> torch.Tensor:
 
 def quantize_mmq_q8_1(x: torch.Tensor, layout: str, k_padded: int | None = None) -> torch.Tensor:
     """`launch_mmq_quantize_q8_1_{D4,DS4}`: x [rows, k] -> uint8 [k_padded / 128, rows, 144]."""
+    k_padded = pad(x.shape[-1], MATRIX_ROW_PADDING) if k_padded is None else k_padded
+    out = kl.host().quantize_mmq_q8_1(x, int(layout == "DS4"), k_padded) if layout in ("D4", "DS4") else None
+    if out is not None:
+        return out
     _require_cuda(x)
     rows, k = x.shape
-    k_padded = pad(pad(k, MATRIX_ROW_PADDING), 128) if k_padded is None else k_padded
     out = torch.empty((k_padded // 128, rows, 144), dtype=torch.uint8, device=x.device)
     fn = getattr(kl.library(), f"launch_mmq_quantize_q8_1_{layout}")
     fn(x.data_ptr(), None, out.data_ptr(), MMQ_TYPE_X[elem_of(x.dtype)], k, k, 0, 0, k_padded, rows, 1, 1, _stream())
@@ -129,8 +147,11 @@ def quantize_mmq_q8_1_glu(gate: torch.Tensor, up: torch.Tensor, layout: str, act
 def mmvq_plain(dtype: GgmlDType, w: torch.Tensor, vy: torch.Tensor, n: int, k: int, b: int,
                out_dtype: torch.dtype, k_padded: int | None = None) -> torch.Tensor:
     """`launch_mmvq_gguf_<type>_<out>_plain` on Q8_1 blocks `vy`; returns [b, n]."""
-    _require_cuda(w, vy)
     k_padded = pad(k, MATRIX_ROW_PADDING) if k_padded is None else k_padded
+    dst = kl.host().mmvq_plain(dtype, w, vy, n, k, b, elem_of(out_dtype), k_padded)
+    if dst is not None:
+        return dst
+    _require_cuda(w, vy)
     dst = torch.empty((b, n), dtype=out_dtype, device=w.device)
     fn = getattr(kl.library(), f"launch_mmvq_gguf_{dtype.tag}_{ELEM_TAG[elem_of(out_dtype)]}_plain")
     fn(w.data_ptr(), vy.data_ptr(), dst.data_ptr(), k, n, k_padded // 32, n, b, _stream())
@@ -147,8 +168,11 @@ def mmvq_fused_glu(dtype: GgmlDType, w_gate: torch.Tensor, w_up: torch.Tensor, v
                    out_dtype: torch.dtype, activation: str = "silu", k_padded: int | None = None) -> torch.Tensor:
     """`launch_mmvq_gguf_<type>_<out>_fused_glu` on Q8_1 blocks `vy`: act(y . gate^T) * (y . up^T), [b, n]
     (fast_mmvq::fused_glu, crates/inference-quant/src/gguf/fast_mmvq.rs)."""
-    _require_cuda(w_gate, w_up, vy)
     k_padded = pad(k, MATRIX_ROW_PADDING) if k_padded is None else k_padded
+    dst = kl.host().mmvq_fused_glu(dtype, w_gate, w_up, vy, n, k, b, elem_of(out_dtype), k_padded, GLU_ACTIVATIONS[activation])
+    if dst is not None:
+        return dst
+    _require_cuda(w_gate, w_up, vy)
     dst = torch.empty((b, n), dtype=out_dtype, device=vy.device)
     name = f"launch_mmvq_gguf_{dtype.tag}_{ELEM_TAG[elem_of(out_dtype)]}_fused_glu"
     getattr(kl.library(), name)(w_gate.data_ptr(), w_up.data_ptr(), vy.data_ptr(), dst.data_ptr(), k, n, k_padded // 32, n, b,
@@ -177,15 +201,25 @@ def mmvq_fused_qkv(dtype: GgmlDType, wq: torch.Tensor, wk: torch.Tensor, wv: tor
 MMQ_LAYOUT = {GgmlDType.Q8_0: "D4", GgmlDType.Q4K: "DS4", GgmlDType.Q6K: "D4"}  # fast_mmq.rs:167-190
 
 
+@functools.lru_cache(maxsize=None)
+def _device_numbers(device: torch.device) -> tuple[int, int]:
+    """The compute capability in the reference's coding, and the number of multiprocessors."""
+    props = torch.cuda.get_device_properties(device)
+    return (props.major * 10 + props.minor) * 10, props.multi_processor_count
+
+
 def mmq(dtype: GgmlDType, w: torch.Tensor, vy: torch.Tensor, m: int, n: int, k: int, out_dtype: torch.dtype) -> torch.Tensor:
     """`launch_mmq_gguf_<type>` on activation blocks `vy` from `quantize_mmq_q8_1(x, MMQ_LAYOUT[dtype])`; returns
     [m, n] of `out_dtype`, called as the reference's host calls it (crates/inference-quant/src/gguf/fast_mmq.rs:489-512)."""
+    cc, nsm = _device_numbers(w.device)
+    dst = kl.host().mmq(dtype, w, vy, m, n, k, elem_of(out_dtype), cc, nsm)
+    if dst is not None:
+        return dst
     _require_cuda(w, vy)
     dst = torch.empty((m, n), dtype=out_dtype, device=w.device)
-    props = torch.cuda.get_device_properties(w.device)
     fn = getattr(kl.library(), f"launch_mmq_gguf_{dtype.tag}")
-    fn(None, w.data_ptr(), vy.data_ptr(), dst.data_ptr(), k, n, m, k // dtype.block_size, n, (props.major * 10 + props.minor) * 10,
-       props.multi_processor_count, 232448, 32, MMQ_TYPE_X[elem_of(out_dtype)], _stream())
+    fn(None, w.data_ptr(), vy.data_ptr(), dst.data_ptr(), k, n, m, k // dtype.block_size, n, cc, nsm, 232448, 32,
+       MMQ_TYPE_X[elem_of(out_dtype)], _stream())
     rc = kl.library().b200q_take_launch_status()
     if rc:
         raise kl.KernelLibraryError(f"launch_mmq_gguf_{dtype.tag} failed with status {rc}")
@@ -249,6 +283,9 @@ def gemv(dtype: GgmlDType, w: torch.Tensor, x: torch.Tensor, n: int, out: torch.
          act_quant: int = ACT_QUANT_Q8_1) -> torch.Tensor:
     """`b200q_gemv`: one launch, activations quantized in the kernel's prologue (to Q8_1, or with
     ``ACT_QUANT_CPU`` to the reference CPU path's Q8_K / Q8_0). x [b, k] -> [b, n] of x's dtype."""
+    dst = kl.host().gemv(dtype, w, x, n, out, act_quant)
+    if dst is not None:
+        return dst
     _require_cuda(w, x)
     b, k = x.shape
     dst = torch.empty((b, n), dtype=x.dtype, device=x.device) if out is None else out
@@ -260,6 +297,9 @@ def gemv(dtype: GgmlDType, w: torch.Tensor, x: torch.Tensor, n: int, out: torch.
 def gemv_group(dtypes, ws, x: torch.Tensor, ns, outs=None, act_quant: int = 0):
     """`b200q_gemv_group` / `b200q_gemv_group_act`: several weight matrices (same K) on one activation row x [1, k] in one
     launch; `act_quant` as for `gemv`."""
+    done = kl.host().gemv_group(dtypes, ws, x, ns, outs, act_quant)
+    if done is not None:
+        return done
     _require_cuda(x, *ws)
     if x.dim() != 2 or x.shape[0] != 1:
         raise ValueError("gemv_group takes a single activation row [1, k]")

@@ -8,12 +8,11 @@ fast_mmq.rs:604-715). Every forward runs the CUDA kernels of the C-ABI library; 
 """
 from __future__ import annotations
 
-import numpy as np
 import torch
 
 from . import ops
 from .dtypes import MATRIX_ROW_PADDING, GgmlDType, pad
-from .kernel_library import KernelLibraryError
+from . import kernel_library as kl
 
 MMVQ_MAX_BATCH = 8  # rows the decode GEMV launchers take (fast_mmvq.rs:84)
 TENSOR_CORE_MAX_ROWS = 16  # rows the small-batch tensor-core kernel takes (fast_mmvq.rs:86)
@@ -27,20 +26,6 @@ def _tensor_core_pays(dtype: GgmlDType, rows: int, n: int, k: int) -> bool:
     if dtype == GgmlDType.Q6K:
         return rows >= 7 or (rows >= 4 and big) or n >= 65536
     return rows >= 5 or big
-
-
-_tc_workspaces: dict = {}
-
-
-def _tc_workspace(dtype: GgmlDType, k: int, device: torch.device) -> torch.Tensor:
-    """One scratch buffer per (device, stream, type, k), like the reference's per-thread, per-stream activation
-    workspace (crates/inference-quant/src/gguf/thread_workspace.rs:94-146): its address is stable, so captured
-    graphs can replay, and calls on one stream are ordered, so they never overlap on it."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream, int(dtype), k)
-    ws = _tc_workspaces.get(key)
-    if ws is None:
-        ws = _tc_workspaces[key] = ops.gemv_tc_workspace(dtype, k, device)
-    return ws
 
 
 def tensor_core_rows_supported(dtype: GgmlDType, k: int) -> bool:
@@ -120,17 +105,22 @@ class QMatMul:
         return cls(qtensor)
 
     def forward(self, xs: torch.Tensor, act_quant: int = ops.ACT_QUANT_Q8_1) -> torch.Tensor:
-        n, k = self.qtensor.shape
+        w = self.qtensor
+        n, k = w.shape
+        y = kl.host().forward(w.dtype, w.data, n, k, xs, act_quant, _tier(w.dtype, xs.numel() // k, n, k, act_quant))
+        if y is not None:
+            return y
+        # whatever the native path declines: errors, empty inputs, and row counts its three kernels do not serve
         if xs.dim() < 2:
             raise ValueError(f"input tensor has only one dimension {tuple(xs.shape)}")
         if not xs.is_contiguous():
             raise ValueError(f"input tensor is not contiguous {tuple(xs.shape)}")
         if xs.shape[-1] != k:
             raise ValueError(f"input tensor {tuple(xs.shape)} incompatible with {(n, k)}")
-        if xs.device != self.qtensor.device:
-            raise ValueError(f"input on {xs.device}, weights on {self.qtensor.device}")
+        if xs.device != w.device:
+            raise ValueError(f"input on {xs.device}, weights on {w.device}")
         x2 = xs.reshape(-1, k)
-        y = _forward_rows(self.qtensor, x2, act_quant)
+        y = _forward_rows(w, x2, act_quant)
         return y.reshape(*xs.shape[:-1], n)
 
     __call__ = forward
@@ -142,33 +132,27 @@ def prefers_mmvq(rows: int) -> bool:
     return rows <= MMVQ_MAX_BATCH
 
 
+def _tier(dtype: GgmlDType, rows: int, n: int, k: int, act_quant: int) -> int:
+    """Which kernel serves a row count: 0 the decode GEMV, 1 the small-batch tensor-core kernel, 2 the tile GEMM."""
+    if rows <= 2:
+        return 0
+    if rows > TENSOR_CORE_MAX_ROWS:
+        return 2
+    if act_quant == ops.ACT_QUANT_Q8_1 and prefers_tensor_core_rows(dtype, rows, n, k):
+        return 1
+    return 0 if prefers_mmvq(rows) else 2
+
+
 def _forward_rows(w: QTensor, x: torch.Tensor, act_quant: int) -> torch.Tensor:
+    """The cases the native path leaves: no rows at all, the CPU format on widths it is not defined for, types the kernels do not
+    take, and wide batches whose K is not a multiple of the tile GEMM's step."""
     n, k = w.shape
     rows = x.shape[0]
     if rows == 0:
         return torch.empty((0, n), dtype=x.dtype, device=x.device)
-    if act_quant == ops.ACT_QUANT_Q8_1 and prefers_tensor_core_rows(w.dtype, rows, n, k):
-        return ops.gemv_tc(w.dtype, w.data, x, n, workspace=_tc_workspace(w.dtype, k, x.device))
+    ops.elem_of(x.dtype)  # raises for a type the kernels do not take
     if prefers_mmvq(rows):
-        if k % 128 == 0:
-            try:
-                return ops.gemv(w.dtype, w.data, x, n, act_quant=act_quant)
-            except KernelLibraryError as exc:
-                # B200Q_ERR_UNSUPPORTED: no staged plan for this call (weights not 16-byte aligned, the simple kernel
-                # forced, no ring that fits). The library can still serve Q8_1 activations in two launches.
-                if act_quant != ops.ACT_QUANT_Q8_1 or exc.status != -1:
-                    raise
-        elif act_quant != ops.ACT_QUANT_Q8_1:
-            raise ValueError(f"the CPU path's activation format needs K a multiple of 128, got {k}")
-        # shapes the one-launch kernel declines: the reference's own two-launch protocol
-        vy = ops.quantize_q8_1(x, pad(k, MATRIX_ROW_PADDING))
-        return ops.mmvq_plain(w.dtype, w.data, vy, n, k, rows, x.dtype)
-    if x.dtype in (torch.bfloat16, torch.float16) and k % 64 == 0:
-        return ops.gemm(w.dtype, w.data, x, n)
-    if x.dtype == torch.float32 and k % 64 == 0:
-        # the tensor-core path takes 16-bit activations; f32 inputs are narrowed as the reference narrows them for
-        # its own CUDA path (crates/inference-quant/src/gguf/mod.rs:667-691 keeps bf16 when given bf16)
-        return ops.gemm(w.dtype, w.data, x.to(torch.bfloat16), n).to(torch.float32)
+        raise ValueError(f"the CPU path's activation format needs K a multiple of 128, got {k}")
     # K not a multiple of 64 (Q8_0 only): batches of the GEMV launcher
     outs = []
     for i in range(0, rows, MMVQ_MAX_BATCH):

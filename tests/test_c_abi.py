@@ -111,3 +111,12 @@ def test_trace_buffer_needs_a_trace_build():
     if rc != 0:
         assert b"B200Q_GEMV_TRACE" in lib.b200q_last_error()
     lib.b200q_set_trace_buffer(None, 0)
+
+
+def test_native_call_path_binds_to_the_library():
+    host = kl.host()
+    assert set(host.symbols()) <= set(kl.SYMBOLS)
+    # arguments it does not take as they stand are declined, never launched
+    assert host.gemv(12, None, None, 16, None, 0) is None
+    assert host.forward(12, None, 16, 256, None, 0, 0) is None
+    assert host.gemv_group([12], [None], None, [16], None, 0) is None
