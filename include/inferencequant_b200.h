@@ -310,6 +310,21 @@ int b200q_gemv_static_scratch(int type, int elem, const void* w, const void* x, 
  * which quantizes activations to Q8_1 blocks and runs launch_mmq_gguf_<type> (ffi.rs:911-927). */
 int b200q_gemm(int type, int elem, const void* w, const void* x, void* y, int M, int N, int K, int ldx, int ldy, void* stream);
 
+/* The same product with a workspace lent for the call (128-byte aligned, b200q_gemm_workspace_bytes bytes; not kept): from the row
+   count on at which it pays, the weights are expanded there once to 16-bit rows and multiplied on CTA pairs
+   (tcgen05 cta_group::2). b200q_gemm_workspace_bytes returns 0 where b200q_gemm is the better call; b200q_gemm_ws then is that
+   call, with or without a workspace. */
+long long b200q_gemm_workspace_bytes(int type, int M, int N, int K);
+int b200q_gemm_ws(int type, int elem, const void* w, const void* x, void* y, int M, int N, int K, int ldx, int ldy, void* workspace,
+                  long long workspace_bytes, void* stream);
+
+/* launch_mmq_gguf_<type> with a workspace lent for the call (128-byte aligned, not kept): act_blocks from
+   launch_mmq_quantize_q8_1_DS4 (Q4_K) or _D4 (Q6_K, Q8_0), y[M][ldy] of element type `elem`, bf16 operands, f32 accumulation.
+   b200q_mmq_workspace_bytes returns 0 for shapes this form does not take. */
+long long b200q_mmq_workspace_bytes(int type, int M, int N, int K);
+int b200q_mmq_ws(int type, int elem, const void* w, const void* act_blocks, void* y, int M, int N, int K, int ldy, void* workspace,
+                 long long workspace_bytes, void* stream);
+
 /* Small batches (M = 1..16 activation rows, B200Q_ERR_TOO_LARGE above) on the tcgen05 tensor cores with 8-bit integer
  * operands: y[M][ldy] = x[M][ldx] . W[N][K]^T, x and y of element type `elem` (f32, f16 or bf16). Two launches on
  * `stream`: x is quantized into `workspace` (int8, one f16-rounded scale d = amax / 127 and the integer sum per 32

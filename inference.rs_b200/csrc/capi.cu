@@ -19,6 +19,10 @@ void gemv_describe(int type, int K, int N, int b, int* out);
 int gemv_group(int elem, int nmat, const int* types, const void* const* ws, void* const* dsts, const int* Ns, int K, const void* x,
                cudaStream_t s, const PeerExchange* px, int act_mode);
 int gemm_dispatch(int type, int elem, const void* w, const void* x, void* y, int M, int N, int K, int ldx, int ldy, cudaStream_t s);
+int gemm_pair_dispatch(int type, int elem, const void* w, const void* x, void* y, int M, int N, int K, int ldx, int ldy, void* workspace, cudaStream_t s);
+size_t gemm_pair_workspace_bytes(int type, int M, int N, int K);
+int mmq_pair_dispatch(int type, int elem, const void* w, const void* aq, void* y, int M, int N, int K, int ldy, void* workspace, cudaStream_t s);
+size_t mmq_pair_workspace_bytes(int type, int M, int N, int K);
 int gemv_tc_dispatch(int type, int elem, const void* w, const void* x, void* y, int M, int N, int K, int ldx, int ldy, void* workspace, cudaStream_t s);
 size_t gemv_tc_workspace_bytes(int type, int K);
 long long peer_allreduce_buffer_bytes(long long capacity);
@@ -56,6 +60,8 @@ int b200q_set_option(const char* name, int value) {
         rt.gemv_stage_target = value;
     } else if (!std::strcmp(name, "tc_ksplit")) {
         rt.tc_ksplit = value ? 1 : 0;
+    } else if (!std::strcmp(name, "gemm_pair_rows")) {
+        rt.gemm_pair_rows = value < 0 ? -1 : value;
     } else if (!std::strcmp(name, "gemm_direct")) {
         rt.gemm_direct = value ? 1 : 0;
     } else if (!std::strcmp(name, "l2_prefetch_bytes")) {
@@ -87,6 +93,7 @@ int b200q_get_option(const char* name, int* value) {
     else if (!std::strcmp(name, "gemv_one_kernel")) *value = rt.gemv_one_kernel;
     else if (!std::strcmp(name, "gemv_passes")) *value = rt.gemv_passes;
     else if (!std::strcmp(name, "gemv_pass_limit_bytes")) *value = rt.gemv_pass_limit;
+    else if (!std::strcmp(name, "gemm_pair_rows")) *value = rt.gemm_pair_rows;
     else if (!std::strcmp(name, "gemm_direct")) *value = rt.gemm_direct;
     else if (!std::strcmp(name, "tc_ksplit")) *value = rt.tc_ksplit;
     else if (!std::strcmp(name, "l2_prefetch_bytes")) *value = l2_prefetch_bytes_effective(rt);
@@ -206,6 +213,48 @@ int b200q_gemm(int type, int elem, const void* w, const void* x, void* y, int M,
         return set_error(rc, "b200q_gemm needs K a multiple of 64 and of the weight type's block size, x 16-byte aligned with ldx * 2 a "
                              "multiple of 16, weights 2-byte aligned (Q4_K: 16-byte), and a driver that provides cuTensorMapEncodeTiled");
     if (rc != 0) return set_error(rc, rc > 0 ? cudaGetErrorString((cudaError_t)rc) : "gemm failed");
+    return B200Q_OK;
+}
+
+// The same product with a workspace of b200q_gemm_workspace_bytes(type, M, N, K) bytes lent for the call: from the row count on at
+// which expanding the weights once pays, they are written there as 16-bit rows and multiplied on CTA pairs (gemm_pair.cu). 0
+// bytes: b200q_gemm is the better call for this shape (and what a call without a workspace runs).
+long long b200q_gemm_workspace_bytes(int type, int M, int N, int K) {
+    if (type_block_bytes(type) == 0 || M <= 0 || N <= 0 || K <= 0 || K % 64 != 0 || K % type_block_elems(type) != 0) return 0;
+    return (long long)gemm_pair_workspace_bytes(type, M, N, K);
+}
+
+int b200q_gemm_ws(int type, int elem, const void* w, const void* x, void* y, int M, int N, int K, int ldx, int ldy, void* workspace,
+                  long long workspace_bytes, void* stream) {
+    const long long need = b200q_gemm_workspace_bytes(type, M, N, K);
+    if (need == 0 || workspace == nullptr) return b200q_gemm(type, elem, w, x, y, M, N, K, ldx, ldy, stream);
+    if (!w || !x || !y) return set_error(B200Q_ERR_INVALID, "null pointer");
+    if (elem != ELEM_BF16 && elem != ELEM_F16) return set_error(B200Q_ERR_UNSUPPORTED, "b200q_gemm_ws takes bf16 or f16 activations");
+    if (workspace_bytes < need) return set_error(B200Q_ERR_INVALID, "workspace smaller than b200q_gemm_workspace_bytes");
+    const int rc = gemm_pair_dispatch(type, elem, w, x, y, M, N, K, ldx, ldy, workspace, (cudaStream_t)stream);
+    if (rc == B200Q_ERR_UNSUPPORTED) return b200q_gemm(type, elem, w, x, y, M, N, K, ldx, ldy, stream);
+    if (rc == B200Q_ERR_INVALID) return set_error(rc, "workspace must be 128-byte aligned");
+    if (rc != 0) return set_error(rc, rc > 0 ? cudaGetErrorString((cudaError_t)rc) : "gemm failed");
+    return B200Q_OK;
+}
+
+// launch_mmq_gguf_* with a workspace lent for the call: activation blocks from launch_mmq_quantize_q8_1_{D4,DS4} (the layout that
+// goes with the weight type), y[M][ldy] of element type `elem`. 0 bytes: shapes this form does not take (use the launcher).
+long long b200q_mmq_workspace_bytes(int type, int M, int N, int K) {
+    if (type_block_bytes(type) == 0 || M <= 0 || N <= 0 || K <= 0 || K % type_block_elems(type) != 0) return 0;
+    return (long long)mmq_pair_workspace_bytes(type, M, N, K);
+}
+
+int b200q_mmq_ws(int type, int elem, const void* w, const void* act_blocks, void* y, int M, int N, int K, int ldy, void* workspace,
+                 long long workspace_bytes, void* stream) {
+    if (!w || !act_blocks || !y || !workspace) return set_error(B200Q_ERR_INVALID, "null pointer");
+    const long long need = b200q_mmq_workspace_bytes(type, M, N, K);
+    if (need == 0) return set_error(B200Q_ERR_UNSUPPORTED, "b200q_mmq_ws needs K a multiple of 256 and packed rows of a multiple of 16 bytes");
+    if (workspace_bytes < need) return set_error(B200Q_ERR_INVALID, "workspace smaller than b200q_mmq_workspace_bytes");
+    const int rc = mmq_pair_dispatch(type, elem, w, act_blocks, y, M, N, K, ldy, workspace, (cudaStream_t)stream);
+    if (rc == B200Q_ERR_UNSUPPORTED) return set_error(rc, "b200q_mmq_ws needs 16-byte aligned weights and blocks");
+    if (rc == B200Q_ERR_INVALID) return set_error(rc, "workspace must be 128-byte aligned");
+    if (rc != 0) return set_error(rc, rc > 0 ? cudaGetErrorString((cudaError_t)rc) : "mmq failed");
     return B200Q_OK;
 }
 

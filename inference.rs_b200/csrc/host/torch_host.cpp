@@ -30,7 +30,9 @@ constexpr int MATRIX_ROW_PADDING = 512;  // activation rows of the two-launch pr
 // ---- the C ABI (include/inferencequant_b200.h) ----
 using GemvFn = int (*)(int, int, const void*, const void*, void*, int, int, int, int, int, int, void*);
 using GroupFn = int (*)(int, const int*, const void* const*, void* const*, const int*, int, int, const void*, int, void*);
-using GemmFn = int (*)(int, int, const void*, const void*, void*, int, int, int, int, int, void*);
+using GemmWsFn = int (*)(int, int, const void*, const void*, void*, int, int, int, int, int, void*, int64_t, void*);
+using MmqWsFn = int (*)(int, int, const void*, const void*, void*, int, int, int, int, void*, int64_t, void*);
+using GemmBytesFn = int64_t (*)(int, int, int, int);
 using GemvTcFn = int (*)(int, int, const void*, const void*, void*, int, int, int, int, int, void*, int64_t, void*);
 using GemvTcBytesFn = int64_t (*)(int, int);
 using QuantizeFn = int (*)(int, const void*, void*, int64_t, void*);
@@ -47,7 +49,9 @@ using MmqFn = void (*)(void*, const void*, const void*, void*, int64_t, int64_t,
 struct Abi {
     GemvFn gemv;
     GroupFn group;
-    GemmFn gemm;
+    GemmWsFn gemm_ws;
+    GemmBytesFn gemm_bytes, mmq_bytes;
+    MmqWsFn mmq_ws;
     GemvTcFn gemv_tc;
     GemvTcBytesFn gemv_tc_bytes;
     QuantizeFn quantize;
@@ -70,7 +74,10 @@ struct AbiEntry {
 const AbiEntry abi_entries[] = {
     {"b200q_gemv", (void**)&abi.gemv},
     {"b200q_gemv_group_act", (void**)&abi.group},
-    {"b200q_gemm", (void**)&abi.gemm},
+    {"b200q_gemm_ws", (void**)&abi.gemm_ws},
+    {"b200q_mmq_ws", (void**)&abi.mmq_ws},
+    {"b200q_mmq_workspace_bytes", (void**)&abi.mmq_bytes},
+    {"b200q_gemm_workspace_bytes", (void**)&abi.gemm_bytes},
     {"b200q_gemv_tc", (void**)&abi.gemv_tc},
     {"b200q_gemv_tc_workspace_bytes", (void**)&abi.gemv_tc_bytes},
     {"b200q_quantize", (void**)&abi.quantize},
@@ -167,6 +174,15 @@ int two_launches(int ti, int elem, const Tensor& w, const Tensor& x, Tensor& y, 
     return launcher_failed("launch_mmvq_gguf_*_plain");
 }
 
+// the tile GEMM; its workspace comes from the caching allocator for the duration of the call (given back in stream order)
+int gemm(long type, int elem, const Tensor& w, const Tensor& x, Tensor& y, int64_t m, int64_t n, int64_t k, int64_t ldx, int64_t ldy) {
+    const int64_t bytes = abi.gemm_bytes((int)type, (int)m, (int)n, (int)k);
+    Tensor ws;
+    if (bytes > 0) ws = empty({bytes}, ScalarType::Byte, x);
+    return call(abi.gemm_ws, (int)type, elem, w.data_ptr(), x.data_ptr(), y.data_ptr(), (int)m, (int)n, (int)k, (int)ldx, (int)ldy,
+                bytes > 0 ? ws.data_ptr() : nullptr, bytes, stream());
+}
+
 // forward(type, w, n, k, x, act_quant, tier): y = x . W^T for contiguous x [..., k]; `tier` is what the caller's routing chose for
 // the row count: 0 decode matvec, 1 small-batch tensor-core kernel, 2 tile GEMM
 PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
@@ -187,9 +203,7 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         // the tensor-core path takes 16-bit activations; f32 inputs are narrowed and the result widened again
         const Tensor x16 = elem == ELEM_F32 ? at::_to_copy(*x, ScalarType::BFloat16) : *x;
         Tensor y = empty(shape, x16.scalar_type(), *x);
-        if (failed(call(abi.gemm, (int)type, elem == ELEM_F32 ? ELEM_BF16 : elem, w->data_ptr(), x16.data_ptr(), y.data_ptr(), (int)rows, (int)n, (int)k, (int)k,
-                            (int)n, stream()),
-                   "b200q_gemm"))
+        if (failed(gemm(type, elem == ELEM_F32 ? ELEM_BF16 : elem, *w, x16, y, rows, n, k, k, n), "b200q_gemm"))
             return nullptr;
         return THPVariable_Wrap(elem == ELEM_F32 ? at::_to_copy(y, ScalarType::Float) : y);
     }
@@ -230,6 +244,21 @@ PyObject* py_gemv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
                         stream()),
                "b200q_gemv"))
         return nullptr;
+    return THPVariable_Wrap(std::move(y));
+    B200Q_CATCH
+}
+
+// gemm(type, w, x, n, out or None)
+PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    B200Q_TRY
+    long type, n;
+    if (nargs != 5 || !int_args(args, {{0, &type}, {3, &n}})) return none();
+    const Tensor *w = tensor_arg(args[1]), *x = tensor_arg(args[2]), *out = args[4] == Py_None ? nullptr : tensor_arg(args[4]);
+    if (!cuda_contiguous(w) || !cuda_contiguous(x) || x->dim() != 2 || (args[4] != Py_None && (out == nullptr || out->dim() != 2))) return none();
+    const int elem = elem_of(x->scalar_type());
+    if (elem < 0) return none();
+    Tensor y = out != nullptr ? *out : empty({x->size(0), n}, x->scalar_type(), *x);
+    if (failed(gemm(type, elem, *w, *x, y, x->size(0), n, x->size(1), x->stride(0), y.stride(0)), "b200q_gemm")) return nullptr;
     return THPVariable_Wrap(std::move(y));
     B200Q_CATCH
 }
@@ -359,6 +388,13 @@ PyObject* py_mmq(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int ti = type_index(type);
     if (ti < 0 || !cuda_contiguous(w) || !cuda_contiguous(vy)) return none();
     Tensor y = empty({m, n}, t, *w);
+    const int64_t bytes = abi.mmq_bytes((int)type, (int)m, (int)n, (int)k);
+    if (bytes > 0) {
+        Tensor ws = empty({bytes}, ScalarType::Byte, *w);
+        const int rc = call(abi.mmq_ws, (int)type, (int)elem, w->data_ptr(), vy->data_ptr(), y.data_ptr(), (int)m, (int)n, (int)k, (int)n, ws.data_ptr(), bytes,
+                            stream());
+        if (rc != ERR_UNSUPPORTED) return failed(rc, "b200q_mmq_ws") ? nullptr : THPVariable_Wrap(std::move(y));
+    }
     call(abi.mmq[ti], nullptr, w->data_ptr(), vy->data_ptr(), y.data_ptr(), k, n, m, k / block_elems(ti), n, (int)cc, (int)nsm, 232448, 32, mmq_type_x((int)elem),
                 stream());
     return launcher_failed("launch_mmq_gguf_*") ? nullptr : THPVariable_Wrap(std::move(y));
@@ -448,6 +484,7 @@ PyMethodDef methods[] = {
     B200Q_FAST("forward", py_forward),
     B200Q_FAST("gemv", py_gemv),
     B200Q_FAST("gemv_group", py_gemv_group),
+    B200Q_FAST("gemm", py_gemm),
     B200Q_FAST("quantize_q8_1", py_quantize_q8_1),
     B200Q_FAST("mmvq_plain", py_mmvq_plain),
     B200Q_FAST("mmvq_fused_glu", py_mmvq_fused_glu),

@@ -10,6 +10,20 @@
 namespace b200q {
 
 // ---- tcgen05 / TMA wrappers ------------------------------------------------------------------
+// One lane of a converged warp. The tensor-core instructions take their descriptors from uniform registers: a loop that the whole
+// warp runs and in which an elected lane issues keeps them there, while a loop inside `if (lane == 0)` holds them per thread and
+// moves them over before every instruction (115-150 cycles between two tcgen05.mma, more than a narrow one takes).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t one;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "elect.sync _|p, 0xffffffff;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(one));
+    return one != 0;
+}
 __device__ __forceinline__ void tma_load_2d(void* dst_smem, const CUtensorMap* map, int x, int y, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(
                      smem_u32(dst_smem)),

@@ -61,6 +61,10 @@ SYMBOLS.update({
     "b200q_set_trace_buffer": ([_vp, _i32], _i32),
     "b200q_gemv": ([_i32, _i32, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i32, _vp], _i32),
     "b200q_gemm": ([_i32, _i32, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp], _i32),
+    "b200q_gemm_workspace_bytes": ([_i32, _i32, _i32, _i32], _i64),
+    "b200q_gemm_ws": ([_i32, _i32, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _i64, _vp], _i32),
+    "b200q_mmq_workspace_bytes": ([_i32, _i32, _i32, _i32], _i64),
+    "b200q_mmq_ws": ([_i32, _i32, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp, _i64, _vp], _i32),
     "b200q_gemv_tc": ([_i32, _i32, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp, _i64, _vp], _i32),
     "b200q_gemv_tc_workspace_bytes": ([_i32, _i32], _i64),
     "b200q_peer_allreduce_buffer_bytes": ([_i64], _i64),

@@ -320,7 +320,10 @@ def gemv_group(dtypes, ws, x: torch.Tensor, ns, outs=None, act_quant: int = 0):
 
 
 def gemm(dtype: GgmlDType, w: torch.Tensor, x: torch.Tensor, n: int, out: torch.Tensor | None = None) -> torch.Tensor:
-    """`b200q_gemm`: prefill tile GEMM on the tensor cores. x [m, k] bf16/f16 -> [m, n] of x's dtype."""
+    """`b200q_gemm_ws`: prefill GEMM on the tensor cores. x [m, k] bf16/f16 -> [m, n] of x's dtype."""
+    y = kl.host().gemm(dtype, w, x, n, out)
+    if y is not None:
+        return y
     _require_cuda(w, x)
     m, k = x.shape
     y = torch.empty((m, n), dtype=x.dtype, device=x.device) if out is None else out

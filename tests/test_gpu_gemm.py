@@ -202,3 +202,25 @@ def test_mmq_launcher_shapes_the_tile_kernel_does_not_take():
 @pytest.mark.parametrize("m", [512, 2048])
 def test_mmq_launcher_prefill_shapes(type_id, k, n, m):
     run_mmq(type_id, m, n, k, packed=real_packed(type_id, n, k), seed=m, real=True, sample_rows=128)
+
+
+# Expanded weights on CTA pairs (b200q_gemm_ws) against the single-launch kernel: the same products in the same order.
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("m,n,k,dtype", [(17, 130, 256, torch.bfloat16), (33, 257, 768, torch.float16), (256, 256, 1280, torch.bfloat16),
+                                         (257, 300, 512, torch.bfloat16), (513, 128, 5120, torch.bfloat16), (1500, 520, 256, torch.float16)])
+def test_workspace_form_equals_the_single_launch(type_id, m, n, k, dtype):
+    if type_id == kq.Q8_0:
+        k += 64  # half a staged chunk: Q8_0 asks for whole steps of 64 only
+    w = ops.upload_weights(random_packed(type_id, n, k, seed=m), DT[type_id])
+    x = seeded_acts(m, k, n, dtype).cuda()
+    rows = ops.get_option("gemm_pair_rows")
+    try:
+        ops.set_option("gemm_pair_rows", 1)
+        pair = ops.gemm(DT[type_id], w, x, n)
+        ops.set_option("gemm_pair_rows", 1 << 30)
+        single = ops.gemm(DT[type_id], w, x, n)
+    finally:
+        ops.set_option("gemm_pair_rows", rows)
+    torch.cuda.synchronize()
+    assert_device_ok()
+    assert torch.equal(pair, single)
