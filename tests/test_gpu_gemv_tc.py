@@ -293,3 +293,21 @@ def test_reference_launcher_pair_on_rows_the_tma_path_cannot_take():
     # Q6_K rows of 210 * k / 256 bytes are a multiple of 16 only when k is a multiple of 2048: other k take the plain kernel
     run_tc_ref(kq.Q6_K, 5, 200, 768, seed=3)
     run_tc_ref(kq.Q6_K, 16, 64, 1280, seed=4)
+
+
+# Tiles of 16 rows in pairs, superblocks shared out over the warps of a pair, K over CTAs where tiles are few: row counts around a tile,
+# a pair and one tile a CTA; one superblock, fewer and more than a CTA has warps, and enough of them for a split along K.
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("m,n,k", [(1, 1, 256), (8, 15, 512), (9, 17, 2048), (16, 33, 8192), (5, 300, 14336), (16, 2373, 1280), (8, 4749, 256)])
+def test_row_tiles_and_superblock_shares(type_id, m, n, k):
+    run_tc(type_id, m, n, k_for(type_id, k), packed=random_packed(type_id, n, k_for(type_id, k), seed=m + n), seed=m)
+
+
+def test_activations_at_any_element_alignment():
+    type_id, n, k = kq.Q4_K, 70, 1024
+    w_dev = ops.upload_weights(random_packed(type_id, n, k, seed=21), DT[type_id])
+    xbig = seeded_acts(9, k + 7, 22, torch.bfloat16).cuda()
+    for off in (0, 1, 2):
+        x = xbig[:, off:off + k]  # rows start on 2-byte boundaries, the row stride is odd
+        assert torch.equal(ops.gemv_tc(DT[type_id], w_dev, x, n), ops.gemv_tc(DT[type_id], w_dev, x.contiguous(), n))
+    assert_device_ok()
