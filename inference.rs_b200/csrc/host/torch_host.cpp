@@ -184,7 +184,7 @@ int gemm(long type, int elem, const Tensor& w, const Tensor& x, Tensor& y, int64
 }
 
 // forward(type, w, n, k, x, act_quant, tier): y = x . W^T for contiguous x [..., k]; `tier` is what the caller's routing chose for
-// the row count: 0 decode matvec, 1 small-batch tensor-core kernel, 2 tile GEMM
+// the row count: 0 decode matvec, 1 small-batch tensor-core kernel, 2 tile GEMM, 3 as 1 or, where that refuses the weights, as 0
 PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     B200Q_TRY
     long type, n, k, act_quant, tier;
@@ -208,15 +208,13 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         return THPVariable_Wrap(elem == ELEM_F32 ? at::_to_copy(y, ScalarType::Float) : y);
     }
     Tensor y = empty(shape, x->scalar_type(), *x);
-    if (tier == 1) {
+    if (tier == 1 || tier == 3) {
         const int64_t bytes = abi.gemv_tc_bytes((int)type, (int)k);
         if (bytes <= 0) return none();
         Tensor ws = empty({bytes}, ScalarType::Byte, *x);  // the allocator reuses it in stream order
-        if (failed(call(abi.gemv_tc, (int)type, elem, w->data_ptr(), x->data_ptr(), y.data_ptr(), (int)rows, (int)n, (int)k, (int)k, (int)n, ws.data_ptr(), bytes,
-                               stream()),
-                   "b200q_gemv_tc"))
-            return nullptr;
-        return THPVariable_Wrap(std::move(y));
+        const int rc = call(abi.gemv_tc, (int)type, elem, w->data_ptr(), x->data_ptr(), y.data_ptr(), (int)rows, (int)n, (int)k, (int)k, (int)n, ws.data_ptr(), bytes,
+                            stream());
+        if (rc != ERR_UNSUPPORTED || tier == 1) return failed(rc, "b200q_gemv_tc") ? nullptr : THPVariable_Wrap(std::move(y));
     }
     if (k % 128 == 0) {
         const int rc = call(abi.gemv, (int)type, elem, w->data_ptr(), x->data_ptr(), y.data_ptr(), (int)k, (int)n, (int)k, (int)n, (int)rows, (int)act_quant, stream());

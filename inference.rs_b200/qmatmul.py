@@ -16,6 +16,7 @@ from . import kernel_library as kl
 
 MMVQ_MAX_BATCH = 8  # rows the decode GEMV launchers take (fast_mmvq.rs:84)
 TENSOR_CORE_MAX_ROWS = 16  # rows the small-batch tensor-core kernel takes (fast_mmvq.rs:86)
+
 # 3..8 rows: the crossovers measured on B200 against the dp4a GEMV at the Llama-3-8B shapes. The tier's cost hardly
 # grows with the row count, the GEMV's grows linearly; Q6_K's unpacking is the most expensive, so it needs more rows
 # or a bigger matrix. 9..16 rows: always (the alternative is the prefill GEMM).
@@ -132,14 +133,29 @@ def prefers_mmvq(rows: int) -> bool:
     return rows <= MMVQ_MAX_BATCH
 
 
+def _tier_overtakes(dtype: GgmlDType, rows: int, n: int, k: int) -> bool:
+    """2..8 rows beyond that rule on which the tier's two launches cost less than the dp4a GEMV, if it takes the weights as they lie.
+    GEMV against tier with weights out of HBM: 2 rows 8.6 / 5.9 us (Q4_K 1024 x 512) to 148 / 85 us (4096 x 128256); 6 rows 10.3 /
+    6.6 us (Q4_K 4096 x 1024), 8.4 / 6.4 us (Q6_K 2048 x 512). In between the GEMV still reads its rows once, and small products
+    favour its shorter prologue: 3 rows of Q4_K 4096 x 1024 6.4 / 6.5 us, 4 rows 7.7 / 6.6; 4 rows of Q6_K 2048 x 4096 7.7 / 7.8,
+    4096 x 4096 13.0 / 10.8."""
+    if not tensor_core_rows_supported(dtype, k):
+        return False
+    return rows == 2 or rows >= 6 or rows * n * k >= (1 << (25 if dtype == GgmlDType.Q6K else 24))
+
+
 def _tier(dtype: GgmlDType, rows: int, n: int, k: int, act_quant: int) -> int:
-    """Which kernel serves a row count: 0 the decode GEMV, 1 the small-batch tensor-core kernel, 2 the tile GEMM."""
-    if rows <= 2:
+    """Which kernel serves a row count: 0 the decode GEMV, 1 the small-batch tensor-core kernel, 2 the tile GEMM, 3 the small-batch
+    kernel or else the GEMV (weights off the 16-byte boundaries that the former needs)."""
+    if rows <= 1:
         return 0
     if rows > TENSOR_CORE_MAX_ROWS:
         return 2
-    if act_quant == ops.ACT_QUANT_Q8_1 and prefers_tensor_core_rows(dtype, rows, n, k):
-        return 1
+    if act_quant == ops.ACT_QUANT_Q8_1:
+        if prefers_tensor_core_rows(dtype, rows, n, k):
+            return 1
+        if prefers_mmvq(rows) and _tier_overtakes(dtype, rows, n, k):
+            return 3
     return 0 if prefers_mmvq(rows) else 2
 
 

@@ -163,6 +163,26 @@ def test_forward_falls_back_to_two_launches_where_the_one_launch_gemv_declines()
     assert_device_ok()
 
 
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("rows,n", [(2, 40), (4, 4096), (6, 40)])
+def test_rows_beyond_the_crossover_agree_with_the_decode_gemv_and_take_weights_at_any_address(type_id, rows, n):
+    # the same integer dot products and scales on both routes, f32 sums in another order: a few of their 2^-24 steps per added block
+    from inference_rs_b200 import ops, qmatmul as qm
+    k, dt = 4096, DT[type_id]
+    assert qm._tier(dt, rows, n, k, ops.ACT_QUANT_Q8_1) == 3 or qm.prefers_tensor_core_rows(dt, rows, n, k)
+    packed = kq.quantize(type_id, seeded_weights(n, k, 52))
+    q = QTensor.from_packed(packed, dt, (n, k))
+    x = seeded_acts(rows, k, 53, torch.float32).cuda()
+    y, want = QMatMul(q).forward(x), ops.gemv(dt, q.data, x, n)
+    atol = 1e-5 * float(want.abs().max())
+    assert (y - want).abs().max().item() <= atol
+    if not qm.prefers_tensor_core_rows(dt, rows, n, k):
+        shifted = torch.empty(q.data.numel() + 2, dtype=torch.uint8, device="cuda")[2:]
+        shifted.copy_(q.data)
+        assert (QMatMul(QTensor(shifted, dt, (n, k))).forward(x) - want).abs().max().item() <= atol
+    assert_device_ok()
+
+
 def test_bias_is_added_after_the_matmul():
     n, k = 32, 256
     packed = kq.quantize(kq.Q8_0, seeded_weights(n, k, 2))
