@@ -81,9 +81,8 @@ template <> struct PairElem<__nv_bfloat16> { static constexpr int format = 1; };
 constexpr int GP_ROWS = 128;      // weight rows of one CTA = TMEM lanes
 constexpr int GP_TOKENS = 256;    // tokens of a tile at most = TMEM columns of one accumulator
 constexpr int GP_BK = 64;         // k per stage: one 128-byte swizzled row of 16-bit elements
-constexpr int GP_STAGES = 6;
+constexpr int GP_MAX_STAGES = 12;
 constexpr int GP_A_BYTES = GP_ROWS * GP_BK * 2;
-constexpr int GP_B_BYTES = GP_TOKENS / 2 * GP_BK * 2;
 constexpr int GP_THREADS = 256;   // warp 0 TMA, warp 1 MMA, warp 2 TMEM, warps 4-7 epilogue
 constexpr int GP_TMEM_COLS = 512; // two accumulators
 
@@ -91,16 +90,17 @@ struct GemmPairParams {
     void* y;  // [M][ldy]
     int M, N, K, ldy;
     int bn;               // tokens per tile: a multiple of 32, <= 256
+    int stages;           // as many as shared memory holds at this bn
     int tiles_m, tiles_n; // token tiles, weight tiles of 256 rows
     unsigned int* status;
 };
 
 struct GemmPairBarriers {
-    uint64_t full[GP_STAGES], empty[GP_STAGES];
+    uint64_t full[GP_MAX_STAGES], empty[GP_MAX_STAGES];
     uint64_t tmem_full[2], tmem_empty[2];
     uint32_t tmem_base;
 };
-constexpr size_t GP_SMEM = 1024 + (size_t)GP_STAGES * (GP_A_BYTES + GP_B_BYTES) + sizeof(GemmPairBarriers);
+constexpr size_t gp_smem(int stages, int bn) { return 1024 + (size_t)stages * (GP_A_BYTES + bn / 2 * GP_BK * 2) + sizeof(GemmPairBarriers); }
 
 template <typename T, typename OutT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
@@ -108,19 +108,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
     extern __shared__ uint8_t gp_smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gp_smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* a_stages = smem;
-    uint8_t* b_stages = smem + GP_STAGES * GP_A_BYTES;
-    GemmPairBarriers* bars = reinterpret_cast<GemmPairBarriers*>(b_stages + GP_STAGES * GP_B_BYTES);
+    const int stages = p.stages, half = p.bn / 2, b_bytes = half * GP_BK * 2;  // bytes: a multiple of 1024
+    uint8_t* b_stages = smem + stages * GP_A_BYTES;
+    GemmPairBarriers* bars = reinterpret_cast<GemmPairBarriers*>(b_stages + stages * b_bytes);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_ctarank();
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
     const int nkb = p.K / GP_BK;
     const int ntiles = p.tiles_m * p.tiles_n;
-    const int half = p.bn / 2;
-    const uint32_t stage_bytes = 2u * (GP_A_BYTES + (uint32_t)half * 128u);  // both CTAs' operands of a stage
+    const uint32_t stage_bytes = 2u * (GP_A_BYTES + (uint32_t)b_bytes);  // both CTAs' operands of a stage
 
     if (tid == 0) {
-        for (int s = 0; s < GP_STAGES; ++s) {
+        for (int s = 0; s < stages; ++s) {
             mbar_init(&bars->full[s], 1);
             mbar_init(&bars->empty[s], 1);
         }
@@ -156,10 +156,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
                 if (elect_one()) {
                     if (rank == 0) mbar_arrive_expect_tx(&bars->full[s], stage_bytes);
                     tma_load_2d_pair(a_stages + (size_t)s * GP_A_BYTES, &tmap_w, kb * GP_BK, row, full0 + 8u * s);
-                    tma_load_2d_pair(b_stages + (size_t)s * GP_B_BYTES, &tmap_x, kb * GP_BK, token, full0 + 8u * s);
+                    tma_load_2d_pair(b_stages + (size_t)s * b_bytes, &tmap_x, kb * GP_BK, token, full0 + 8u * s);
                 }
                 __syncwarp();
-                if (++s == GP_STAGES) {
+                if (++s == stages) {
                     s = 0;
                     ph ^= 1u;
                 }
@@ -168,8 +168,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
         // the leader waits for its last copies before the CTAs may exit (they are counted on its barriers; the MMAs have
         // consumed them unless something gave up)
         if (!ok && rank == 0) {
-            for (int q = 0; q < min(g, GP_STAGES); ++q) {
-                if (s == 0) { s = GP_STAGES - 1; ph ^= 1u; } else --s;
+            for (int q = 0; q < min(g, stages); ++q) {
+                if (s == 0) { s = stages - 1; ph ^= 1u; } else --s;
                 if (!mbar_wait_bounded(&bars->full[s], ph ^ 1u)) {
                     if (lane == 0) record_failure(p.status, STATUS_WAIT_DRAIN_TIMEOUT, q);
                     break;
@@ -200,7 +200,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
                         break;
                     }
                     tc_fence_after();
-                    const uint64_t da = da0 + (uint64_t)(s * (GP_A_BYTES >> 4)), db = db0 + (uint64_t)(s * (GP_B_BYTES >> 4));
+                    const uint64_t da = da0 + (uint64_t)(s * (GP_A_BYTES >> 4)), db = db0 + (uint64_t)(s * (b_bytes >> 4));
                     if (elect_one()) {
 #pragma unroll
                         for (int k = 0; k < GP_BK / 16; ++k) tc_mma_f16_pair(d, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
@@ -208,7 +208,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GP_THREADS, 1)
                         if (kb == nkb - 1) tc_commit_pair(&bars->tmem_full[buf]);
                     }
                     __syncwarp();
-                    if (++s == GP_STAGES) {
+                    if (++s == stages) {
                         s = 0;
                         ph ^= 1u;
                     }
@@ -384,6 +384,31 @@ static cudaError_t expand_weights(int type, const void* w, T* out, long long val
     return launch_expand<TYPE_Q8_0, T>(w, out, values, s);
 }
 
+// Tokens per tile. Tiles go out in waves of one per CTA pair, and a wave takes as long as its tile is high, but no less than a tile of
+// about 148 tokens (an MMA of 256 rows has a floor near 64 cycles; K = 4096: 12.5 us a wave up to 160 tokens, 15.5 at 192, 21 at
+// 256). So the height is the one with the least waves x height, plus some 24 tokens' worth a wave for filling and draining; as few
+// tiles as 256 tokens allow unless that is beaten by 5 % (more tiles read the weights again from L2). Against always the fewest:
+// 512 x 4096 x 14336 (32 tiles for 74 pairs -> 64) 95 -> 77 us, 1024 x 14336 x 4096 (224 tiles in 4 waves -> 280 in 4) 121 -> 111,
+// 1024 x 6144 x 4096 57 -> 48, 333 x 6144 x 4096 32.7 -> 31.3.
+static int token_tile(int M, int tiles_n) {
+    const int pairs = runtime_info().sm_count / 2;
+    long long best = 0;
+    int best_bn = 0;
+    for (int tm = (M + GP_TOKENS - 1) / GP_TOKENS, last = 0;; ++tm) {
+        const int bn = (((M + tm - 1) / tm) + 31) & ~31;
+        if (best_bn != 0 && bn < 128) break;
+        if (bn == last) continue;
+        last = bn;
+        const long long waves = ((long long)((M + bn - 1) / bn) * tiles_n + pairs - 1) / pairs;
+        const long long cost = waves * ((bn > 148 ? bn : 148) + 24);
+        if (best_bn == 0 || cost * 100 < best * 95) {
+            best = cost;
+            best_bn = bn;
+        }
+    }
+    return best_bn;
+}
+
 template <typename T, typename OutT>
 static int launch_pair(const T* w16, const T* x, void* y, int M, int N, int K, int ldx, int ldy, cudaStream_t s, bool dependent) {
     GemmPairParams p{};
@@ -393,9 +418,9 @@ static int launch_pair(const T* w16, const T* x, void* y, int M, int N, int K, i
     p.K = K;
     p.ldy = ldy;
     p.status = status_ptr();
-    // token tiles of equal height, as few as 256 tokens a tile allow
-    const int tm = (M + GP_TOKENS - 1) / GP_TOKENS;
-    p.bn = (((M + tm - 1) / tm) + 31) & ~31;
+    p.bn = token_tile(M, (N + 2 * GP_ROWS - 1) / (2 * GP_ROWS));
+    p.stages = GP_MAX_STAGES;
+    while (gp_smem(p.stages, p.bn) > (size_t)runtime_info().smem_optin - 1024) --p.stages;
     p.tiles_m = (M + p.bn - 1) / p.bn;
     p.tiles_n = (N + 2 * GP_ROWS - 1) / (2 * GP_ROWS);
     const CUtensorMapDataType dt = PairElem<T>::format == 1 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -418,7 +443,7 @@ static int launch_pair(const T* w16, const T* x, void* y, int M, int N, int K, i
     cudaError_t e = allow_full_smem<kernel>();
     if (e != cudaSuccess) return (int)e;
     const int ntiles = p.tiles_m * p.tiles_n, pairs = runtime_info().sm_count / 2;
-    e = launch_dependent(kernel, 2u * (unsigned)(ntiles < pairs ? ntiles : pairs), GP_THREADS, GP_SMEM, s, dependent, map_w, map_x, p);
+    e = launch_dependent(kernel, 2u * (unsigned)(ntiles < pairs ? ntiles : pairs), GP_THREADS, gp_smem(p.stages, p.bn), s, dependent, map_w, map_x, p);
     return (int)e;
 }
 

@@ -224,3 +224,10 @@ def test_workspace_form_equals_the_single_launch(type_id, m, n, k, dtype):
     torch.cuda.synchronize()
     assert_device_ok()
     assert torch.equal(pair, single)
+
+
+# Token tiles lower than 256 where that saves a wave of tiles: counts on both sides of the rule's choices, ragged last tiles.
+@pytest.mark.parametrize("m,n,k,dtype", [(333, 6144, 256, torch.bfloat16), (512, 4096, 512, torch.float16), (700, 14336, 256, torch.bfloat16),
+                                         (1025, 6100, 256, torch.bfloat16)])
+def test_token_tile_heights_equal_the_single_launch(m, n, k, dtype):
+    test_workspace_form_equals_the_single_launch(kq.Q4_K, m, n, k, dtype)
