@@ -330,13 +330,13 @@ int b200q_mmq_ws(int type, int elem, const void* w, const void* act_blocks, void
  * `stream`: x is quantized into `workspace` (int8, one f16-rounded scale d = amax / 127 and the integer sum per 32
  * values: the layout kernel mmvq_tc_quantize of the reference, mmvq_gguf/mmvq_quantize.cu:157-190, computes the same
  * values), then one persistent CTA per SM streams its share of the packed weight rows once, unpacks them to int8 and
- * multiplies 128 rows x 32 k blocks by all rows of x with tcgen05.mma kind::i8; block scales are applied in f32.
+ * multiplies them block by block by all rows of x with mma.sync (int8); block scales are applied in f32.
  * Takes the place of the reference's tensor-core matvec tier for 2..16 rows: fast_mmvq::tiled_plain
  * (crates/inference-quant/src/gguf/fast_mmvq.rs:2049-2126) with launch_mmvq_tc_quantize_<elem> +
  * launch_mmvq_tc_gguf_<type>_<elem>_plain (ffi.rs:631-652,954-998; kernel mmvq_gguf/mmvq_tc_k.cuh:221-329).
  * Needs K a multiple of 256, w 16-byte aligned with a row size that is a multiple of 16 bytes (Q6_K: K a multiple of
  * 2048), workspace 128-byte aligned and at least b200q_gemv_tc_workspace_bytes(type, K) bytes (0 = unsupported K;
- * 18 K bytes, 34 K for Q6_K, plus 1.3 MB for the partial outputs of matrices that are split along K);
+ * 24 K bytes plus 164 KB for the partial outputs of matrices that are split along K);
  * the workspace is the caller's, as the reference's activation scratch is (gguf/thread_workspace.rs:94-146), and
  * must not be shared by calls that can overlap on the GPU. */
 long long b200q_gemv_tc_workspace_bytes(int type, int K);
