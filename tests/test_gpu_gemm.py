@@ -231,3 +231,25 @@ def test_workspace_form_equals_the_single_launch(type_id, m, n, k, dtype):
                                          (1025, 6100, 256, torch.bfloat16)])
 def test_token_tile_heights_equal_the_single_launch(m, n, k, dtype):
     test_workspace_form_equals_the_single_launch(kq.Q4_K, m, n, k, dtype)
+
+
+# Packed rows of Q8_0 and Q6_K staged by 16-byte loads: a last piece that is not a whole CTA's, and weights on any even address.
+@pytest.mark.parametrize("type_id", [kq.Q8_0, kq.Q6_K])
+@pytest.mark.parametrize("n,k,off", [(33, 256, 0), (131, 768, 2), (64, 1280, 14)])
+def test_expansion_of_ragged_pieces_and_even_addresses(type_id, n, k, off):
+    packed = random_packed(type_id, n, k, seed=n)
+    w = ops.upload_weights(packed, DT[type_id])
+    shifted = torch.empty(w.numel() + off, dtype=torch.uint8, device="cuda")[off:]
+    shifted.copy_(w)
+    x = seeded_acts(300, k, n, torch.bfloat16).cuda()
+    rows = ops.get_option("gemm_pair_rows")
+    try:
+        ops.set_option("gemm_pair_rows", 1)
+        pair = ops.gemm(DT[type_id], shifted, x, n)
+        ops.set_option("gemm_pair_rows", 1 << 30)
+        single = ops.gemm(DT[type_id], w, x, n)
+    finally:
+        ops.set_option("gemm_pair_rows", rows)
+    torch.cuda.synchronize()
+    assert_device_ok()
+    assert torch.equal(pair, single)
