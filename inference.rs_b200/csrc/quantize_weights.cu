@@ -62,7 +62,9 @@ __global__ void __launch_bounds__(256) quantize_q8_0_kernel(const float* __restr
             for (int i = 0; i < 4; ++i) v[i] = xb[i];
         }
     }
-    float amax = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+    float amax = 0.0f;  // and not v[0]: fmaxf passes a NaN over, so a block of nothing else has the scale 0
+#pragma unroll
+    for (int i = 0; i < 4; ++i) amax = fmaxf(amax, fabsf(v[i]));
 #pragma unroll
     for (int m = 4; m > 0; m >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, m));
     const float d = amax / 127.0f;

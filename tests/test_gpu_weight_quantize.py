@@ -157,3 +157,17 @@ def test_dequantize_rows_of_any_width_and_alignment(type_id, n, k):
         got = out.cpu().numpy()
         assert np.array_equal(got[o_off // 4:o_off // 4 + n * k].reshape(n, k), want)
         assert not got[:o_off // 4].any() and not got[o_off // 4 + n * k:].any()
+
+
+def test_q8_0_blocks_with_nan_and_infinite_values():
+    """The reference's maximum starts from 0 and passes NaNs over (quantized/mod.rs:43-56): a block of NaNs alone has the scale 0."""
+    w = seeded_weights(2, 160, 31)
+    w[0, :32] = np.nan
+    w[0, 32:36] = np.nan
+    w[0, 64] = np.inf
+    w[0, 96:127] = np.nan
+    w[1, 5] = -np.inf
+    w[1, 128:] = np.nan
+    got = ops.quantize_weights(torch.from_numpy(w).cuda(), DT[kq.Q8_0])
+    want = kq.quantize(kq.Q8_0, w).reshape(-1)
+    assert np.array_equal(got.cpu().numpy()[: want.size], want)
