@@ -114,9 +114,11 @@ __global__ void __launch_bounds__(128) tcq_quantize_kernel(const src_t* __restri
             tcq_load4<src_t>(p, vec, v);
             tcq_load4<src_t>(p + 16, vec, v + 4);
         }
-        float amax = 0.0f;
+        // from the first value on, as the reference's warp maximum: a NaN among other values counts as 0, but a block of NaNs alone has
+        // a NaN for a scale and makes its row's outputs NaNs
+        float amax = fabsf(v[0]);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+        for (int i = 1; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         const float d = amax / 127.0f;

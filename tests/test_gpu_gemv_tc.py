@@ -311,3 +311,27 @@ def test_activations_at_any_element_alignment():
         x = xbig[:, off:off + k]  # rows start on 2-byte boundaries, the row stride is odd
         assert torch.equal(ops.gemv_tc(DT[type_id], w_dev, x, n), ops.gemv_tc(DT[type_id], w_dev, x.contiguous(), n))
     assert_device_ok()
+
+
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("m", [8, 12])
+def test_blocks_of_nans_and_infinities_reach_the_outputs(type_id, m):
+    """As in the reference's quantizer (mmvq_quantize.cu:157-190): a block of NaNs alone or with an infinity gives a NaN row, a NaN
+    among other values counts as 0, and the other rows do not change."""
+    n, k = 70, k_for(type_id, 1024)
+    w_dev = ops.upload_weights(random_packed(type_id, n, k, seed=31), DT[type_id])
+    clean = seeded_acts(m, k, 32, torch.float32)
+    clean[3, 5] = 0.0
+    x = clean.clone()
+    x[2, 64:96] = float("nan")
+    x[3, 5] = float("nan")
+    x[4, 40] = float("inf")
+    x[5] = float("nan")
+    want, y = ops.gemv_tc(DT[type_id], w_dev, clean.cuda(), n), ops.gemv_tc(DT[type_id], w_dev, x.cuda(), n)
+    lost = torch.zeros(m, dtype=torch.bool)
+    lost[[2, 4, 5]] = True
+    assert bool(y[lost.cuda()].isnan().all()) and torch.equal(y[~lost.cuda()], want[~lost.cuda()])
+    if type_id != kq.Q8_0:
+        pair = ops.mmvq_tc_plain(DT[type_id], w_dev, ops.mmvq_tc_quantize(x.cuda()), n, k, m, torch.float32)
+        assert torch.equal(pair.isnan(), y.isnan())
+    assert_device_ok()
