@@ -115,14 +115,16 @@ void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 // ---- arguments ----
 const Tensor* tensor_arg(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 bool cuda_contiguous(const Tensor* t) { return t != nullptr && t->is_cuda() && t->is_contiguous(); }
+// anything that counts as an integer (a numpy integer has an index too)
 bool int_arg(PyObject* o, long& v) {
-    if (!PyLong_Check(o)) return false;
-    v = PyLong_AsLong(o);
-    if (v == -1 && PyErr_Occurred()) {
-        PyErr_Clear();
-        return false;
+    PyObject* i = PyNumber_Index(o);
+    if (i != nullptr) {
+        v = PyLong_AsLong(i);
+        Py_DECREF(i);
     }
-    return true;
+    if (i != nullptr && !(v == -1 && PyErr_Occurred())) return true;
+    PyErr_Clear();
+    return false;
 }
 bool int_args(PyObject* const* args, std::initializer_list<std::pair<int, long*>> list) {
     for (const auto& [i, v] : list)
@@ -283,8 +285,9 @@ PyObject* py_gemv_group(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     Tensor outs[MAX];
     for (Py_ssize_t i = 0; i < n; ++i) {
         long t, rows;
+        if (!int_arg(PySequence_Fast_GET_ITEM(args[0], i), t) || !int_arg(PySequence_Fast_GET_ITEM(args[3], i), rows)) return none();
         const Tensor* w = tensor_arg(PySequence_Fast_GET_ITEM(args[1], i));
-        if (!cuda_contiguous(w) || !int_arg(PySequence_Fast_GET_ITEM(args[0], i), t) || !int_arg(PySequence_Fast_GET_ITEM(args[3], i), rows)) return none();
+        if (!cuda_contiguous(w)) return none();
         types[i] = (int)t;
         ns[i] = (int)rows;
         ws[i] = w->data_ptr();

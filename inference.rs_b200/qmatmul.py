@@ -46,7 +46,7 @@ class QTensor:
     """Packed GGUF blocks of a `[n, k]` weight on a CUDA device (rows contiguous, then the reference's padding)."""
 
     def __init__(self, data: torch.Tensor, dtype: GgmlDType, shape: tuple[int, int]):
-        n, k = shape
+        n, k = int(shape[0]), int(shape[1])  # a shape read through numpy holds numpy integers
         if k % dtype.block_size:
             # mod.rs:872-884: the last dimension must hold whole blocks
             raise ValueError(f"quantized tensor last dim {k} is not a multiple of the {dtype.name} block size {dtype.block_size}")
@@ -111,7 +111,7 @@ class QMatMul:
         y = kl.host().forward(w.dtype, w.data, n, k, xs, act_quant, _tier(w.dtype, xs.numel() // k, n, k, act_quant))
         if y is not None:
             return y
-        # whatever the native path declines: errors, empty inputs, and row counts its three kernels do not serve
+        # what the native path declines as it stands: errors among them
         if xs.dim() < 2:
             raise ValueError(f"input tensor has only one dimension {tuple(xs.shape)}")
         if not xs.is_contiguous():
@@ -160,22 +160,42 @@ def _tier(dtype: GgmlDType, rows: int, n: int, k: int, act_quant: int) -> int:
 
 
 def _forward_rows(w: QTensor, x: torch.Tensor, act_quant: int) -> torch.Tensor:
-    """The cases the native path leaves: no rows at all, the CPU format on widths it is not defined for, types the kernels do not
-    take, and wide batches whose K is not a multiple of the tile GEMM's step."""
+    """The same kernels by the same rule where the native path declines a call: empty inputs, wide batches whose K is not a multiple
+    of the tile GEMM's step, the CPU format on widths it is not defined for, and whatever the kernels' own checks refuse."""
     n, k = w.shape
     rows = x.shape[0]
     if rows == 0:
         return torch.empty((0, n), dtype=x.dtype, device=x.device)
-    ops.elem_of(x.dtype)  # raises for a type the kernels do not take
-    if prefers_mmvq(rows):
+    tier = _tier(w.dtype, rows, n, k, act_quant)
+    if tier in (1, 3):
+        try:
+            return ops.gemv_tc(w.dtype, w.data, x, n)
+        except kl.KernelLibraryError as exc:
+            if tier == 1 or exc.status != -1:  # -1: weights off the 16-byte boundaries
+                raise
+    if tier == 2 and k % 64 == 0:
+        if x.dtype == torch.float32:
+            # the tensor-core path takes 16-bit activations; f32 inputs are narrowed as the reference narrows them for
+            # its own CUDA path (crates/inference-quant/src/gguf/mod.rs:667-691 keeps bf16 when given bf16)
+            return ops.gemm(w.dtype, w.data, x.to(torch.bfloat16), n).to(torch.float32)
+        return ops.gemm(w.dtype, w.data, x, n)
+    if tier != 2 and k % 128 == 0:
+        try:
+            return ops.gemv(w.dtype, w.data, x, n, act_quant=act_quant)
+        except kl.KernelLibraryError as exc:
+            # no staged plan for this call (weights not 16-byte aligned, the simple kernel forced, no ring that fits): the
+            # library can still serve Q8_1 activations in two launches
+            if act_quant != ops.ACT_QUANT_Q8_1 or exc.status != -1:
+                raise
+    elif tier != 2 and act_quant != ops.ACT_QUANT_Q8_1:
         raise ValueError(f"the CPU path's activation format needs K a multiple of 128, got {k}")
-    # K not a multiple of 64 (Q8_0 only): batches of the GEMV launcher
+    # the reference's own two-launch protocol, in batches of its launcher
     outs = []
     for i in range(0, rows, MMVQ_MAX_BATCH):
         xb = x[i:i + MMVQ_MAX_BATCH].contiguous()
         vy = ops.quantize_q8_1(xb, pad(k, MATRIX_ROW_PADDING))
         outs.append(ops.mmvq_plain(w.dtype, w.data, vy, n, k, xb.shape[0], x.dtype))
-    return torch.cat(outs, 0)
+    return outs[0] if len(outs) == 1 else torch.cat(outs, 0)
 
 
 class GgufMatMul:

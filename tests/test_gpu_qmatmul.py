@@ -183,6 +183,20 @@ def test_rows_beyond_the_crossover_agree_with_the_decode_gemv_and_take_weights_a
     assert_device_ok()
 
 
+@pytest.mark.parametrize("type_id", TYPES)
+def test_shapes_read_through_numpy_are_shapes(type_id):
+    from inference_rs_b200 import kernel_library as kl, ops
+    n, k, dt = 48, 512, DT[type_id]
+    q = QTensor.from_packed(kq.quantize(type_id, seeded_weights(n, k, 54)), dt, (n, k))
+    like_numpy = QTensor(q.data, dt, tuple(np.array([n, k], dtype=np.int32)))
+    for rows in (1, 4, 12, 40):
+        x = seeded_acts(rows, k, 55, torch.bfloat16).cuda()
+        assert torch.equal(QMatMul(like_numpy).forward(x), QMatMul(q).forward(x))
+        if rows <= 8:
+            assert torch.equal(kl.host().gemv(dt, q.data, x, np.int64(n), None, np.int64(0)), ops.gemv(dt, q.data, x, n))
+    assert_device_ok()
+
+
 def test_bias_is_added_after_the_matmul():
     n, k = 32, 256
     packed = kq.quantize(kq.Q8_0, seeded_weights(n, k, 2))
