@@ -465,14 +465,28 @@ static int launch_pair(const T* w16, const T* x, void* y, int M, int N, int K, i
     return (int)e;
 }
 
-// Where the single-launch kernel of gemm_tcgen05.cu stays: up to 256 rows on matrices tall enough to give every SM a tile of it
-// (it then expands no weight twice and saves the 16-bit copy: 256 x 28672 x 4096 Q4_K 100 us against 130 us; but 128 x 4096 x 4096
-// Q6_K 60 us against 40 us), and only where it can stage packed rows in shared memory. From 257 rows on it expands twice or more.
+// Where the single-launch kernel of gemm_tcgen05.cu stays: it expands each weight tile in the CTA that multiplies it, so with one tile
+// of tokens it expands nothing twice and saves the 16-bit copy, but a tile of 128 weight rows takes an SM the same time however many
+// SMs have one. So it stays where it can stage packed rows in shared memory and
+//   * every SM has a tile, up to 256 rows (256 x 28672 x 4096 Q4_K 84 us against 106 us; one row more doubles its time), or
+//   * up to 128 rows (its tile of tokens), where enough SMs have one. Where the two meet, of 148 tiles, us single / pair at 17 and 128
+//     rows: Q4_K K = 4096 88 tiles 39.7 / 36.0, 40.7 / 37.7, 96 39.7 / 38.8, 41.4 / 41.7, 112 39.8 / 44.2, 41.2 / 47.1, K = 14336 88
+//     125 / 124, 127 / 127; Q8_0 K = 4096 104 47.0 / 48.0, 48.3 / 49.3, K = 14336 96 151 / 148, 153 / 152; Q6_K, slower to unpack,
+//     K = 4096 120 52.0 / 52.9, 53.4 / 54.2, K = 14336 112 167 / 168, 169 / 170. Narrower matrices have less to expand: K = 2048 at 128
+//     rows, 128 tiles, Q4_K 23.3 / 25.1, Q8_0 27.1 / 28.9, but Q6_K 29.8 / 27.7.
+// From 257 rows on it expands twice or more and is the slower one everywhere.
 static bool gemm_pair_pays(int type, int M, int N, int K) {
     const int rows = runtime_info().gemm_pair_rows;
     if (rows >= 0) return M >= rows;
     const bool staged = K % 256 == 0 && (long long)K / type_block_elems(type) * type_block_bytes(type) % 16 == 0;
-    return !staged || M > 256 || (N + 127) / 128 < runtime_info().sm_count;
+    if (!staged || M > 256) return true;
+    const int tiles = (N + 127) / 128, sms = runtime_info().sm_count;
+    if (tiles >= sms) return false;
+    if (M > 128) return true;
+    // of 148 tiles: 93 / 99 / 111 and more stay (Q4_K / Q8_0 / Q6_K), at narrower K 124 / 124 / 148
+    const bool wide = K >= 3072;
+    const int twenty_fourths = type == TYPE_Q4_K ? (wide ? 15 : 20) : (type == TYPE_Q8_0 ? (wide ? 16 : 20) : (wide ? 18 : 24));
+    return 24 * tiles < twenty_fourths * sms;
 }
 size_t gemm_pair_workspace_bytes(int type, int M, int N, int K) { return gemm_pair_pays(type, M, N, K) ? (size_t)N * K * 2 : 0; }
 // quantized activations: their 16-bit copy as well. The single-launch kernel expands them in every tile, so this pays wherever that

@@ -120,3 +120,21 @@ def test_native_call_path_binds_to_the_library():
     assert host.gemv(12, None, None, 16, None, 0) is None
     assert host.forward(12, None, 16, 256, None, 0, 0) is None
     assert host.gemv_group([12], [None], None, [16], None, 0) is None
+
+
+def test_the_expanded_form_is_chosen_where_it_is_not_slower():
+    """b200q_gemm_workspace_bytes: 0 = the single launch. Up to 128 rows it stays where enough SMs have a tile of 128 weight rows (the
+    measured crossovers, of 148 SMs), up to 256 where every SM has one."""
+    lib = pkg.library()
+    q8, q4, q6 = 8, 12, 14
+    pair = lambda t, m, n, k: lib.b200q_gemm_workspace_bytes(t, m, n, k) > 0
+    for t, k, n in ((q4, 4096, 11776), (q8, 4096, 12672), (q6, 4096, 14208), (q4, 2048, 15744), (q8, 512, 15744), (q6, 2048, 18816)):
+        assert lib.b200q_gemm_workspace_bytes(t, 128, n, k) in (0, 2 * n * k)
+        assert pair(t, 17, n - 256, k) and pair(t, 128, n - 256, k), (t, n, k)
+        assert not pair(t, 17, n + 128, k) and not pair(t, 128, n + 128, k), (t, n, k)
+        assert pair(t, 257, n + 128, k) and pair(t, 8192, n, k)
+    for t in (q8, q4, q6):
+        assert pair(t, 129, 18816, 4096) and not pair(t, 256, 18945, 4096) and pair(t, 257, 28672, 4096)
+    # rows that cannot be staged are expanded by every tile from byte loads: the single launch is the slower one at any size
+    assert pair(q8, 17, 28672, 4160) and pair(q6, 17, 28672, 5120)
+    assert lib.b200q_gemm_workspace_bytes(q4, 40, 64, 100) == 0
