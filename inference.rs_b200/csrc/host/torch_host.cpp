@@ -11,10 +11,10 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/_to_copy.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>  // C++ exceptions become the Python ones torch raises itself (OutOfMemoryError among them)
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
-#include <exception>
 #include <initializer_list>
 
 namespace {
@@ -158,14 +158,6 @@ int launcher_failed(const char* what) {
     return 1;
 }
 
-#define B200Q_TRY try {
-#define B200Q_CATCH                                      \
-    }                                                    \
-    catch (const std::exception& e) {                    \
-        PyErr_SetString(PyExc_RuntimeError, e.what());   \
-        return nullptr;                                  \
-    }
-
 // ---- matmul ----
 // quantize to Q8_1, then the reference's own matvec: shapes the one-launch kernel declines
 int two_launches(int ti, int elem, const Tensor& w, const Tensor& x, Tensor& y, int64_t n, int64_t k, int64_t rows) {
@@ -188,7 +180,7 @@ int gemm(long type, int elem, const Tensor& w, const Tensor& x, Tensor& y, int64
 // forward(type, w, n, k, x, act_quant, tier): y = x . W^T for contiguous x [..., k]; `tier` is what the caller's routing chose for
 // the row count: 0 decode matvec, 1 small-batch tensor-core kernel, 2 tile GEMM, 3 as 1 or, where that refuses the weights, as 0
 PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type, n, k, act_quant, tier;
     if (nargs != 7 || !int_args(args, {{0, &type}, {2, &n}, {3, &k}, {5, &act_quant}, {6, &tier}})) return none();
     const Tensor *w = tensor_arg(args[1]), *x = tensor_arg(args[4]);
@@ -226,12 +218,12 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         return none();
     }
     return two_launches(ti, elem, *w, *x, y, n, k, rows) ? nullptr : THPVariable_Wrap(std::move(y));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // gemv(type, w, x, n, out or None, act_quant)
 PyObject* py_gemv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type, n, act_quant;
     if (nargs != 6 || !int_args(args, {{0, &type}, {3, &n}, {5, &act_quant}})) return none();
     const Tensor *w = tensor_arg(args[1]), *x = tensor_arg(args[2]), *out = args[4] == Py_None ? nullptr : tensor_arg(args[4]);
@@ -245,12 +237,12 @@ PyObject* py_gemv(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
                "b200q_gemv"))
         return nullptr;
     return THPVariable_Wrap(std::move(y));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // gemm(type, w, x, n, out or None)
 PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type, n;
     if (nargs != 5 || !int_args(args, {{0, &type}, {3, &n}})) return none();
     const Tensor *w = tensor_arg(args[1]), *x = tensor_arg(args[2]), *out = args[4] == Py_None ? nullptr : tensor_arg(args[4]);
@@ -260,12 +252,12 @@ PyObject* py_gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     Tensor y = out != nullptr ? *out : empty({x->size(0), n}, x->scalar_type(), *x);
     if (failed(gemm(type, elem, *w, *x, y, x->size(0), n, x->size(1), x->stride(0), y.stride(0)), "b200q_gemm")) return nullptr;
     return THPVariable_Wrap(std::move(y));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // gemv_group(types, ws, x, ns, outs or None, act_quant): lists of 1..4
 PyObject* py_gemv_group(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     constexpr int MAX = 4;
     long act_quant;
     if (nargs != 6 || !int_arg(args[5], act_quant)) return none();
@@ -311,13 +303,13 @@ PyObject* py_gemv_group(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     PyObject* list = PyList_New(n);
     for (Py_ssize_t i = 0; list != nullptr && i < n; ++i) PyList_SET_ITEM(list, i, THPVariable_Wrap(std::move(outs[i])));
     return list;
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // ---- the reference host's own sequence ----
 // quantize_q8_1(x, k_padded)
 PyObject* py_quantize_q8_1(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long kp;
     if (nargs != 2 || !int_arg(args[1], kp)) return none();
     const Tensor* x = tensor_arg(args[0]);
@@ -325,7 +317,7 @@ PyObject* py_quantize_q8_1(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     Tensor out = empty({x->size(0), kp / 32 * 36}, ScalarType::Byte, *x);
     call(abi.quant_q8[elem_of(x->scalar_type())], x->data_ptr(), out.data_ptr(), (int)x->size(1), (int)kp, (int)x->size(0), stream());
     return THPVariable_Wrap(std::move(out));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // elem code of an output type given as its code
@@ -337,7 +329,7 @@ bool elem_scalar(long elem, ScalarType& t) {
 
 // mmvq_plain(type, w, vy, n, k, b, elem, k_padded)
 PyObject* py_mmvq_plain(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type, n, k, b, elem, kp;
     ScalarType t;
     if (nargs != 8 || !int_args(args, {{0, &type}, {3, &n}, {4, &k}, {5, &b}, {6, &elem}, {7, &kp}}) || !elem_scalar(elem, t)) return none();
@@ -347,12 +339,12 @@ PyObject* py_mmvq_plain(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     Tensor y = empty({b, n}, t, *w);
     call(abi.plain[ti][elem], w->data_ptr(), vy->data_ptr(), y.data_ptr(), (int)k, (int)n, (int)(kp / 32), (int)n, (int)b, stream());
     return launcher_failed("launch_mmvq_gguf_*_plain") ? nullptr : THPVariable_Wrap(std::move(y));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // mmvq_fused_glu(type, w_gate, w_up, vy, n, k, b, elem, k_padded, activation)
 PyObject* py_mmvq_fused_glu(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type, n, k, b, elem, kp, act;
     ScalarType t;
     if (nargs != 10 || !int_args(args, {{0, &type}, {4, &n}, {5, &k}, {6, &b}, {7, &elem}, {8, &kp}, {9, &act}}) || !elem_scalar(elem, t)) return none();
@@ -362,12 +354,12 @@ PyObject* py_mmvq_fused_glu(PyObject*, PyObject* const* args, Py_ssize_t nargs) 
     Tensor y = empty({b, n}, t, *vy);
     call(abi.glu[ti][elem], wg->data_ptr(), wu->data_ptr(), vy->data_ptr(), y.data_ptr(), (int)k, (int)n, (int)(kp / 32), (int)n, (int)b, (int)act, stream());
     return launcher_failed("launch_mmvq_gguf_*_fused_glu") ? nullptr : THPVariable_Wrap(std::move(y));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // quantize_mmq_q8_1(x, ds4, k_padded)
 PyObject* py_quantize_mmq_q8_1(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long ds4, kp;
     if (nargs != 3 || !int_args(args, {{1, &ds4}, {2, &kp}})) return none();
     const Tensor* x = tensor_arg(args[0]);
@@ -376,12 +368,12 @@ PyObject* py_quantize_mmq_q8_1(PyObject*, PyObject* const* args, Py_ssize_t narg
     Tensor out = empty({kp / 128, rows, 144}, ScalarType::Byte, *x);
     call(abi.quant_mmq[ds4 ? 1 : 0], x->data_ptr(), nullptr, out.data_ptr(), mmq_type_x(elem_of(x->scalar_type())), k, k, 0, 0, kp, rows, 1, 1, stream());
     return THPVariable_Wrap(std::move(out));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // mmq(type, w, vy, m, n, k, elem, cc, nsm)
 PyObject* py_mmq(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type, m, n, k, elem, cc, nsm;
     ScalarType t;
     if (nargs != 9 || !int_args(args, {{0, &type}, {3, &m}, {4, &n}, {5, &k}, {6, &elem}, {7, &cc}, {8, &nsm}}) || !elem_scalar(elem, t)) return none();
@@ -399,13 +391,13 @@ PyObject* py_mmq(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     call(abi.mmq[ti], nullptr, w->data_ptr(), vy->data_ptr(), y.data_ptr(), k, n, m, k / block_elems(ti), n, (int)cc, (int)nsm, 232448, 32, mmq_type_x((int)elem),
                 stream());
     return launcher_failed("launch_mmq_gguf_*") ? nullptr : THPVariable_Wrap(std::move(y));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // ---- weights ----
 // quantize(type, x): f32 [n, k] -> packed blocks, then the padding, zeroed
 PyObject* py_quantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type;
     if (nargs != 2 || !int_arg(args[0], type)) return none();
     const Tensor* x = tensor_arg(args[1]);
@@ -416,12 +408,12 @@ PyObject* py_quantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     buf.narrow(0, bytes, padding).zero_();
     if (failed(call(abi.quantize, (int)type, x->data_ptr(), buf.data_ptr(), x->numel(), stream()), "b200q_quantize")) return nullptr;
     return THPVariable_Wrap(std::move(buf));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // dequantize(type, w, n, k, elem)
 PyObject* py_dequantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type, n, k, elem;
     ScalarType t;
     if (nargs != 5 || !int_args(args, {{0, &type}, {2, &n}, {3, &k}, {4, &elem}}) || !elem_scalar(elem, t)) return none();
@@ -430,12 +422,12 @@ PyObject* py_dequantize(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     Tensor out = empty({n, k}, t, *w);
     if (failed(call(abi.dequantize, (int)type, (int)elem, w->data_ptr(), out.data_ptr(), n, (int)k, stream()), "b200q_dequantize")) return nullptr;
     return THPVariable_Wrap(std::move(out));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // get_rows(type, w, ids, n, k, elem): ids int32, contiguous, on the device
 PyObject* py_get_rows(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
-    B200Q_TRY
+    HANDLE_TH_ERRORS
     long type, n, k, elem;
     ScalarType t;
     if (nargs != 6 || !int_args(args, {{0, &type}, {3, &n}, {4, &k}, {5, &elem}}) || !elem_scalar(elem, t)) return none();
@@ -448,7 +440,7 @@ PyObject* py_get_rows(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
                "b200q_get_rows"))
         return nullptr;
     return THPVariable_Wrap(std::move(out));
-    B200Q_CATCH
+    END_HANDLE_TH_ERRORS
 }
 
 // bind(names, addresses, check, launch_failed)

@@ -1,4 +1,5 @@
 """GPU tests of the host-side operator mirror (`QMatMul`, `GgufMatMul`) and of the tensor-parallel layers."""
+import contextlib
 import os
 import socket
 
@@ -194,6 +195,32 @@ def test_shapes_read_through_numpy_are_shapes(type_id):
         assert torch.equal(QMatMul(like_numpy).forward(x), QMatMul(q).forward(x))
         if rows <= 8:
             assert torch.equal(kl.host().gemv(dt, q.data, x, np.int64(n), None, np.int64(0)), ops.gemv(dt, q.data, x, n))
+    assert_device_ok()
+
+
+@contextlib.contextmanager
+def device_memory_left(nbytes):
+    """At most nbytes more for torch's allocator."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + nbytes) / total)
+    try:
+        yield
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def test_running_out_of_memory_keeps_its_type():
+    from inference_rs_b200 import ops
+    n, k, dt = 8192, 8192, DT[kq.Q8_0]
+    q = QTensor(torch.zeros(n * dt.row_bytes(k), dtype=torch.uint8, device="cuda"), dt, (n, k))
+    x = torch.zeros(4096, k, dtype=torch.bfloat16, device="cuda")
+    with device_memory_left(32 << 20):
+        for call in (lambda: q.dequantize(), lambda: QMatMul(q).forward(x), lambda: ops.gemm(dt, q.data, x, n)):
+            with pytest.raises(torch.OutOfMemoryError):
+                call()
+    assert not q.dequantize().any()
     assert_device_ok()
 
 
