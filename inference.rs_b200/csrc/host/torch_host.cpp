@@ -168,17 +168,27 @@ int two_launches(int ti, int elem, const Tensor& w, const Tensor& x, Tensor& y, 
     return launcher_failed("launch_mmvq_gguf_*_plain");
 }
 
-// the tile GEMM; its workspace comes from the caching allocator for the duration of the call (given back in stream order)
+// A workspace from the caching allocator for the duration of a call (given back in stream order); undefined if none is needed or the
+// memory is not there, where the caller has a form that needs none.
+Tensor workspace(int64_t bytes, const Tensor& like) {
+    if (bytes <= 0) return Tensor();
+    try {
+        return empty({bytes}, ScalarType::Byte, like);
+    } catch (const c10::OutOfMemoryError&) {
+        return Tensor();
+    }
+}
+
+// the tile GEMM
 int gemm(long type, int elem, const Tensor& w, const Tensor& x, Tensor& y, int64_t m, int64_t n, int64_t k, int64_t ldx, int64_t ldy) {
     const int64_t bytes = abi.gemm_bytes((int)type, (int)m, (int)n, (int)k);
-    Tensor ws;
-    if (bytes > 0) ws = empty({bytes}, ScalarType::Byte, x);
+    const Tensor ws = workspace(bytes, x);
     return call(abi.gemm_ws, (int)type, elem, w.data_ptr(), x.data_ptr(), y.data_ptr(), (int)m, (int)n, (int)k, (int)ldx, (int)ldy,
-                bytes > 0 ? ws.data_ptr() : nullptr, bytes, stream());
+                ws.defined() ? ws.data_ptr() : nullptr, bytes, stream());
 }
 
 // forward(type, w, n, k, x, act_quant, tier): y = x . W^T for contiguous x [..., k]; `tier` is what the caller's routing chose for
-// the row count: 0 decode matvec, 1 small-batch tensor-core kernel, 2 tile GEMM, 3 as 1 or, where that refuses the weights, as 0
+// the row count: 0 decode matvec, 1 small-batch tensor-core kernel, 2 tile GEMM, 3 as 1 or, where that refuses the weights or finds no room for its workspace, as 0
 PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     long type, n, k, act_quant, tier;
@@ -205,9 +215,10 @@ PyObject* py_forward(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (tier == 1 || tier == 3) {
         const int64_t bytes = abi.gemv_tc_bytes((int)type, (int)k);
         if (bytes <= 0) return none();
-        Tensor ws = empty({bytes}, ScalarType::Byte, *x);  // the allocator reuses it in stream order
-        const int rc = call(abi.gemv_tc, (int)type, elem, w->data_ptr(), x->data_ptr(), y.data_ptr(), (int)rows, (int)n, (int)k, (int)k, (int)n, ws.data_ptr(), bytes,
-                            stream());
+        const Tensor ws = tier == 1 ? empty({bytes}, ScalarType::Byte, *x) : workspace(bytes, *x);
+        const int rc = !ws.defined() ? ERR_UNSUPPORTED
+                                     : call(abi.gemv_tc, (int)type, elem, w->data_ptr(), x->data_ptr(), y.data_ptr(), (int)rows, (int)n, (int)k, (int)k, (int)n,
+                                            ws.data_ptr(), bytes, stream());
         if (rc != ERR_UNSUPPORTED || tier == 1) return failed(rc, "b200q_gemv_tc") ? nullptr : THPVariable_Wrap(std::move(y));
     }
     if (k % 128 == 0) {
@@ -382,8 +393,7 @@ PyObject* py_mmq(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (ti < 0 || !cuda_contiguous(w) || !cuda_contiguous(vy)) return none();
     Tensor y = empty({m, n}, t, *w);
     const int64_t bytes = abi.mmq_bytes((int)type, (int)m, (int)n, (int)k);
-    if (bytes > 0) {
-        Tensor ws = empty({bytes}, ScalarType::Byte, *w);
+    if (const Tensor ws = workspace(bytes, *w); ws.defined()) {
         const int rc = call(abi.mmq_ws, (int)type, (int)elem, w->data_ptr(), vy->data_ptr(), y.data_ptr(), (int)m, (int)n, (int)k, (int)n, ws.data_ptr(), bytes,
                             stream());
         if (rc != ERR_UNSUPPORTED) return failed(rc, "b200q_mmq_ws") ? nullptr : THPVariable_Wrap(std::move(y));

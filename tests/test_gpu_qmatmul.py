@@ -224,6 +224,26 @@ def test_running_out_of_memory_keeps_its_type():
     assert_device_ok()
 
 
+@pytest.mark.parametrize("type_id", TYPES)
+def test_prompt_products_need_no_memory_beside_their_output(type_id):
+    """The 16-bit copy of the weights (2 n k bytes) is an option: where it does not fit, the form without it runs, same products in the
+    same order."""
+    from inference_rs_b200 import ops
+    n, k, m, dt = 16384, 8192, 300, DT[type_id]
+    q = QTensor.quantize(torch.randn(n, k, device="cuda", generator=torch.Generator("cuda").manual_seed(1)), dt)
+    x = seeded_acts(m, k, 56, torch.bfloat16).cuda()
+    vy = ops.quantize_mmq_q8_1(x, ops.MMQ_LAYOUT[dt])
+    assert pkg.library().b200q_gemm_workspace_bytes(int(dt), m, n, k) == 2 * n * k
+    assert pkg.library().b200q_mmq_workspace_bytes(int(dt), m, n, k) >= 2 * n * k
+    calls = (lambda: QMatMul(q).forward(x), lambda: ops.gemm(dt, q.data, x, n), lambda: ops.mmq(dt, q.data, vy, m, n, k, x.dtype))
+    for call in calls:
+        want = call()
+        with device_memory_left(64 << 20):
+            got = call()
+        assert torch.equal(got, want)
+    assert_device_ok()
+
+
 def test_bias_is_added_after_the_matmul():
     n, k = 32, 256
     packed = kq.quantize(kq.Q8_0, seeded_weights(n, k, 2))
