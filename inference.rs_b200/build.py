@@ -71,25 +71,40 @@ def _compile(nvcc: str, src: str, obj: str, extra: list[str]) -> tuple[str, str]
     return src, res.stdout + res.stderr
 
 
-def build_host(force: bool = False, verbose: bool = False) -> str:
-    """The torch front end's native call path (a CPython extension against this interpreter's torch), if anything changed."""
+def _torch_dir() -> str | None:
     import importlib.util
+
+    spec = importlib.util.find_spec("torch")
+    return next(iter(spec.submodule_search_locations)) if spec is not None else None
+
+
+def build_host(force: bool = False, verbose: bool = False) -> str | None:
+    """The torch front end's native call path (a CPython extension against this interpreter's torch), if anything changed. None where
+    there is no such torch or nothing to compile an extension with: a host of the C library needs neither."""
     import sysconfig
 
-    torch_dir = next(iter(importlib.util.find_spec("torch").submodule_search_locations))
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DAT_PER_OPERATOR_HEADERS",
-           f"-I{torch_dir}/include", f"-I{torch_dir}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}",
-           f"-I{os.path.dirname(os.path.dirname(_nvcc()))}/include", HOST_SRC, f"-L{torch_dir}/lib",
-           "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
-    h = hashlib.sha256(repr(cmd).encode() + sys.version.encode())
+    torch_dir, python_include = _torch_dir(), sysconfig.get_paths()["include"]
+    if torch_dir is None or not os.path.exists(os.path.join(torch_dir, "lib", "libc10_cuda.so")):
+        if verbose:
+            print("no torch with CUDA: its call path is not built", file=sys.stderr)
+        return None
+    flags = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DAT_PER_OPERATOR_HEADERS",
+             f"-I{torch_dir}/include", f"-I{torch_dir}/include/torch/csrc/api/include", f"-I{python_include}"]
+    libs = [f"-L{torch_dir}/lib", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10"]
+    h = hashlib.sha256(repr((flags, libs)).encode() + sys.version.encode())
     for path in (HOST_SRC, os.path.join(torch_dir, "version.py")):
         with open(path, "rb") as fh:
             h.update(fh.read())
     digest_file = HOST_LIB + ".digest"
     if not force and os.path.exists(HOST_LIB) and os.path.exists(digest_file) and open(digest_file).read() == h.hexdigest():
         return HOST_LIB
+    if shutil.which("g++") is None or not os.path.exists(os.path.join(python_include, "Python.h")):
+        if verbose:
+            print("no g++ or no Python headers: torch's call path is not built", file=sys.stderr)
+        return None
+    cuda_include = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
     os.makedirs(os.path.dirname(HOST_LIB), exist_ok=True)
-    res = subprocess.run([*cmd, "-o", HOST_LIB + ".tmp"], capture_output=True, text=True)
+    res = subprocess.run(["g++", *flags, f"-I{cuda_include}", HOST_SRC, *libs, "-o", HOST_LIB + ".tmp"], capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"g++ failed for {HOST_SRC}:\n{res.stdout}\n{res.stderr}")
     os.replace(HOST_LIB + ".tmp", HOST_LIB)
@@ -101,8 +116,14 @@ def build_host(force: bool = False, verbose: bool = False) -> str:
 
 
 def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
-    """Build the shared library (and the torch front end's native part) if any source changed; return its path."""
+    """Build the shared library, then the torch front end's native part, if any source changed; return the library's path."""
+    lib = build_library(force, verbose, ptxas_info)
     build_host(force, verbose)
+    return lib
+
+
+def build_library(force: bool = False, verbose: bool = False, ptxas_info: bool = False) -> str:
+    """Build the C library if any source changed; return its path."""
     hdr = _headers_digest()
     # one digest over every source: a library built from these exact sources is reused even where the object
     # directory did not travel with it
