@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_NAME = "libinferencequant_b200.so"
@@ -131,21 +132,38 @@ def library() -> C.CDLL:
 _host = None
 
 
+class NoNativePath:
+    """Stands in for the native call path: declines every call, so that the Python forms in ops.py and qmatmul.py make it."""
+
+    def __getattr__(self, name):
+        return self._decline
+
+    @staticmethod
+    def _decline(*args):
+        return None
+
+
 def host():
-    """The torch front end's native call path (csrc/host/torch_host.cpp), bound to `library()`; raises KernelLibraryError if it
-    was not built."""
+    """The torch front end's native call path (csrc/host/torch_host.cpp), bound to `library()`. Where it was not built, or not for this
+    torch, calls go through their Python forms, which launch the same kernels 15-20 us of host time later; a warning says so once."""
     global _host
     if _host is None:
         from importlib.machinery import ExtensionFileLoader
         from importlib.util import module_from_spec, spec_from_file_location
-        path = os.path.join(HERE, "lib", HOST_LIB_NAME)
-        if not os.path.exists(path):
-            raise KernelLibraryError(f"{path} not found; build it with `python inference.rs_b200/build.py`.")
-        name = HOST_LIB_NAME.split(".")[0]
-        spec = spec_from_file_location(name, path, loader=ExtensionFileLoader(name, path))
-        mod = module_from_spec(spec)
-        spec.loader.exec_module(mod)
         lib = library()
+        path = os.path.join(HERE, "lib", HOST_LIB_NAME)
+        name = HOST_LIB_NAME.split(".")[0]
+        try:
+            if not os.path.exists(path):
+                raise ImportError(f"{path} not found")
+            spec = spec_from_file_location(name, path, loader=ExtensionFileLoader(name, path))
+            mod = module_from_spec(spec)
+            spec.loader.exec_module(mod)
+        except ImportError as exc:
+            warnings.warn(f"native call path not available ({exc}); calls go through Python. Build it with `python inference.rs_b200/build.py`.",
+                          RuntimeWarning, stacklevel=2)
+            _host = NoNativePath()
+            return _host
         mod.bind({sym: C.cast(getattr(lib, sym), _vp).value for sym in mod.symbols()}, check, launch_failed)
         _host = mod
     return _host

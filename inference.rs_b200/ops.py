@@ -2,7 +2,7 @@
 
 Every function launches on torch's current CUDA stream and raises if the kernel library is unavailable. The functions of the
 matmul path hand their arguments to the native call path (csrc/host/torch_host.cpp); what it does not take as it stands it
-declines with None, and the Python form below it raises the error or deals with the case.
+declines with None, and the Python form below it raises the error or makes the call (all calls, where that path is not built).
 """
 from __future__ import annotations
 
@@ -88,9 +88,12 @@ def get_rows(dtype: GgmlDType, w: torch.Tensor, ids: torch.Tensor, n: int, k: in
     if out is not None:
         return out
     _require_cuda(w)
-    out = kl.host().get_rows(dtype, w, ids.to(device=w.device, dtype=torch.int32).contiguous(), n, k, elem)
+    ids = ids.to(device=w.device, dtype=torch.int32).contiguous()
+    out = kl.host().get_rows(dtype, w, ids, n, k, elem)
     if out is None:
-        raise TypeError("get_rows takes packed weights and integer ids")
+        out = torch.empty((*ids.shape, k), dtype=out_dtype, device=w.device)
+        kl.check(kl.library().b200q_get_rows(int(dtype), elem, w.data_ptr(), ids.data_ptr(), out.data_ptr(), ids.numel(), k, n, _stream()),
+                 "b200q_get_rows")
     return out
 
 

@@ -138,3 +138,16 @@ def test_the_expanded_form_is_chosen_where_it_is_not_slower():
     # rows that cannot be staged are expanded by every tile from byte loads: the single launch is the slower one at any size
     assert pair(q8, 17, 28672, 4160) and pair(q6, 17, 28672, 5120)
     assert lib.b200q_gemm_workspace_bytes(q4, 40, 64, 100) == 0
+
+
+@pytest.mark.parametrize("content", [None, b"not a library"])
+def test_without_the_native_call_path_calls_are_left_to_python(monkeypatch, tmp_path, content):
+    kl.library()
+    monkeypatch.setattr(kl, "_host", None)
+    monkeypatch.setattr(kl, "HERE", str(tmp_path))
+    if content is not None:
+        (tmp_path / "lib").mkdir()
+        (tmp_path / "lib" / kl.HOST_LIB_NAME).write_bytes(content)
+    with pytest.warns(RuntimeWarning, match="native call path"):
+        host = kl.host()
+    assert kl.host() is host and host.forward(1, 2) is None and host.gemv() is None

@@ -198,6 +198,43 @@ def test_shapes_read_through_numpy_are_shapes(type_id):
     assert_device_ok()
 
 
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_python_forms_of_the_calls_give_the_native_paths_results(monkeypatch, type_id, dtype):
+    from inference_rs_b200 import kernel_library as kl, ops
+    n, k, dt = 300, 2048, DT[type_id]
+    assert not isinstance(kl.host(), kl.NoNativePath)
+    w = torch.from_numpy(seeded_weights(n, k, 57)).cuda()
+    ids = torch.tensor([[5, 0, 299]], dtype=torch.int64)
+
+    def everything():
+        q = QTensor.quantize(w, dt)
+        outs = [q.data, q.dequantize(dtype), q.embedding(ids, dtype), q.embedding(ids.cuda().int(), dtype)]
+        for rows in (1, 2, 7, 12, 40, 300):
+            x = seeded_acts(rows, k, 58, dtype).cuda()
+            outs += [QMatMul(q).forward(x), QMatMul(q).forward(x[None])]
+            if rows <= 8:
+                vy = ops.quantize_q8_1(x)
+                outs += [ops.gemv(dt, q.data, x, n), ops.gemv(dt, q.data, x, n, act_quant=ops.ACT_QUANT_CPU), vy,
+                         ops.mmvq_plain(dt, q.data, vy, n, k, rows, dtype), ops.mmvq_fused_glu(dt, q.data, q.data, vy, n, k, rows, dtype)]
+            else:
+                vy = ops.quantize_mmq_q8_1(x, ops.MMQ_LAYOUT[dt])
+                outs += [vy, ops.mmq(dt, q.data, vy, rows, n, k, dtype)]
+            if rows == 1:
+                outs += ops.gemv_group([dt, dt], [q.data, q.data], x, [n, 100])
+            if rows > 8 and dtype == torch.bfloat16:
+                outs.append(ops.gemm(dt, q.data, x, n))
+        return outs
+
+    native = everything()
+    monkeypatch.setattr(kl, "_host", kl.NoNativePath())
+    python = everything()
+    assert len(native) == len(python)
+    for i, (a, b) in enumerate(zip(native, python)):
+        assert a.dtype == b.dtype and torch.equal(a, b), i
+    assert_device_ok()
+
+
 @contextlib.contextmanager
 def device_memory_left(nbytes):
     """At most nbytes more for torch's allocator."""
