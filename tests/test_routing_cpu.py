@@ -84,3 +84,11 @@ def test_tensors_off_the_gpu_are_named_as_the_error(rows):
     q = QTensor(torch.zeros(16 * 144, dtype=torch.uint8), GgmlDType.Q4K, (16, 256))
     with pytest.raises(ValueError, match="CUDA tensor"):
         QMatMul(q).forward(torch.zeros(rows, 256, dtype=torch.bfloat16))
+
+
+def test_launchers_name_tensors_off_the_gpu_as_the_error():
+    w, acts = torch.zeros(16 * 144, dtype=torch.uint8), torch.zeros(2, 20, 144, dtype=torch.uint8)
+    with pytest.raises(ValueError, match="CUDA tensor"):
+        qm.ops.mmq(GgmlDType.Q4K, w, acts, 20, 16, 256, torch.bfloat16)
+    with pytest.raises(ValueError, match="CUDA tensor"):
+        qm.ops.quantize_mmq_q8_1(torch.zeros(20, 256), "DS4")
