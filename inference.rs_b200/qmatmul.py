@@ -135,13 +135,28 @@ def prefers_mmvq(rows: int) -> bool:
 
 def _tier_overtakes(dtype: GgmlDType, rows: int, n: int, k: int) -> bool:
     """2..8 rows beyond that rule on which the tier's two launches cost less than the dp4a GEMV, if it takes the weights as they lie.
-    GEMV against tier with weights out of HBM: 2 rows 8.6 / 5.9 us (Q4_K 1024 x 512) to 148 / 85 us (4096 x 128256); 6 rows 10.3 /
-    6.6 us (Q4_K 4096 x 1024), 8.4 / 6.4 us (Q6_K 2048 x 512). In between the GEMV still reads its rows once, and small products
-    favour its shorter prologue: 3 rows of Q4_K 4096 x 1024 6.4 / 6.5 us, 4 rows 7.7 / 6.6; 4 rows of Q6_K 2048 x 4096 7.7 / 7.8,
-    4096 x 4096 13.0 / 10.8."""
+    The tier takes 6 us at least and hardly grows with the rows; the GEMV starts at 3.3 and grows with rows * n * k, the faster the
+    wider the rows are. GEMV / tier, us, weights out of HBM, on both sides of the lines: Q4_K k = 1024 3 rows 12288 7.45 / 7.70, 16384
+    8.56 / 8.19, 4 rows 8192 6.66 / 7.19, 12288 8.46 / 7.76; k = 2048 3 rows 4096 6.40 / 7.00, 8192 8.90 / 8.41; k = 4096 3 rows 1024
+    6.50 / 6.57, 2048 7.89 / 6.90. Q8_0 k = 1024 3 rows 12288 8.52 / 9.00, 16384 10.0 / 9.65; k = 4096 3 rows 1024 6.84 / 8.21, 2048
+    8.13 / 7.94; even counts cost its GEMV more, 4 rows k = 512 12288 6.15 / 6.95, k = 1024 4096 6.03 / 6.33, 6144 6.92 / 6.84. Q6_K k =
+    2048 3 rows 8192 9.80 / 10.9, 12288 13.0 / 12.9, 5 rows 1024 6.24 / 6.42, 4096 8.97 / 7.84; k = 4096 3 rows 2048 8.12 / 8.33, 4096
+    10.7 / 10.7. 2 rows, at any size: Q4_K 8.10 / 5.99 (512 x 256) to 79 / 48 (4096 x 65536), Q8_0 7.10 / 5.90 (256 x 256) to 171 / 77
+    (6144 x 65536), Q6_K 10.9 / 6.25 (2048 x 256) to 201 / 97; 6 rows of Q6_K 8.67 / 6.33 to 354 / 98."""
     if not tensor_core_rows_supported(dtype, k):
         return False
-    return rows == 2 or rows >= 6 or rows * n * k >= (1 << (25 if dtype == GgmlDType.Q6K else 24))
+    if rows == 2 or rows >= 6:
+        return True
+    narrow = k < 3072
+    if dtype == GgmlDType.Q6K:
+        least = 9 if narrow and rows < 5 else 4
+    elif dtype == GgmlDType.Q4K:
+        least = 5 if narrow else 2
+    elif rows == 3:
+        least = 5 if narrow else 3
+    else:
+        least = 5 if k < 1024 else (3 if k < 1536 else 2)
+    return rows * n * k >= least << 23
 
 
 def _tier(dtype: GgmlDType, rows: int, n: int, k: int, act_quant: int) -> int:

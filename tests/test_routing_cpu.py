@@ -92,3 +92,26 @@ def test_launchers_name_tensors_off_the_gpu_as_the_error():
         qm.ops.mmq(GgmlDType.Q4K, w, acts, 20, 16, 256, torch.bfloat16)
     with pytest.raises(ValueError, match="CUDA tensor"):
         qm.ops.quantize_mmq_q8_1(torch.zeros(20, 256), "DS4")
+
+
+# (type, rows, k, rows of the matrix at which the GEMV is still the faster one, at which the tier is): measured on B200
+@pytest.mark.parametrize("dtype,rows,k,gemv,tier", [
+    (GgmlDType.Q4K, 3, 512, 16383, 16384), (GgmlDType.Q4K, 3, 1024, 12288, 16384), (GgmlDType.Q4K, 4, 1024, 8192, 12288),
+    (GgmlDType.Q4K, 3, 2048, 4096, 8192), (GgmlDType.Q4K, 4, 2048, 2048, 6144), (GgmlDType.Q4K, 3, 4096, 1024, 2048),
+    (GgmlDType.Q8_0, 4, 512, 12288, 16384), (GgmlDType.Q8_0, 3, 1024, 12288, 16384), (GgmlDType.Q8_0, 4, 1024, 4096, 6144),
+    (GgmlDType.Q8_0, 3, 4096, 1024, 2048), (GgmlDType.Q6K, 3, 2048, 8192, 12288), (GgmlDType.Q6K, 4, 2048, 6144, 12288),
+    (GgmlDType.Q6K, 5, 2048, 1024, 4096), (GgmlDType.Q6K, 3, 4096, 2048, 4096)])
+def test_3_to_5_rows_leave_the_gemv_where_the_tier_is_not_slower(dtype, rows, k, gemv, tier):
+    assert qm._tier(dtype, rows, gemv, k, qm.ops.ACT_QUANT_Q8_1) == 0
+    assert qm._tier(dtype, rows, tier, k, qm.ops.ACT_QUANT_Q8_1) in (1, 3)
+
+
+@pytest.mark.parametrize("dtype", [GgmlDType.Q4K, GgmlDType.Q6K, GgmlDType.Q8_0])
+def test_the_kernel_of_each_row_count(dtype):
+    q8_1, cpu = qm.ops.ACT_QUANT_Q8_1, qm.ops.ACT_QUANT_CPU
+    for k, n in LLAMA_SHAPES:
+        assert [qm._tier(dtype, r, n, k, q8_1) for r in (1, 2)] == [0, 3]
+        assert all(qm._tier(dtype, r, n, k, q8_1) in (1, 3) for r in range(6, 9)) and {qm._tier(dtype, r, n, k, q8_1) for r in range(9, 17)} == {1}
+        assert qm._tier(dtype, 17, n, k, q8_1) == 2
+        assert [qm._tier(dtype, r, n, k, cpu) for r in (2, 8, 9)] == [0, 0, 2]
+    assert qm._tier(dtype, 2, 4096, 4096 + 128, q8_1) == 0 and qm._tier(dtype, 12, 4096, 4096 + 128, q8_1) == 2
