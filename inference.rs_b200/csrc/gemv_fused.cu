@@ -55,7 +55,7 @@ struct GemvGluParams {
 
 // One CTA per SM, 16 consumer warps + 1 producer warp, as gemv_staged_kernel; NREG = register-resident item slots.
 template <int TYPE, int B, typename dst_t, int NREG>
-__global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_glu_kernel(GemvGluParams p) {
+__global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_glu_kernel(const GemvGluParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     uint64_t* full = reinterpret_cast<uint64_t*>(smem);
     uint64_t* empty = full + GEMV_MAX_STAGES;
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 1) gemv_glu_kernel(GemvGluParams
     }
 }
 
-// Shapes the ring kernel does not take (K not a multiple of 128, unaligned weights, no ring that fits): a warp per row,
+// Shapes the ring kernel does not take (K not a multiple of 128, unaligned weights, no ring that fits) or is slower on (small Q8_0): a warp per row,
 // byte-granular loads, both dot products per 32-value group.
 template <int TYPE, int B, typename dst_t>
 __global__ void __launch_bounds__(256) gemv_glu_simple_kernel(const uint8_t* __restrict__ wg, const uint8_t* __restrict__ wu,
@@ -372,6 +372,13 @@ static int launch_glu_b(const void* wg, const void* wu, const void* vy, void* ds
         }
         ring_ok = S >= 2;
         p.nstages = S;
+        // Small matrices of the type that needs no unpacking, where a stage holds less than a pass, so that some warps stay idle: the
+        // plain kernel below, a warp per row, until its CTAs come in several waves or its rows are long. Plain / ring, us, Q8_0: 1 row
+        // 512 x 256 2.6 / 3.7, 2048 x 256 2.9 / 3.5, 1000 x 1024 3.2 / 3.9, 1536 x 1024 4.7 / 4.2; 2 rows 512 x 256 3.1 / 5.5, 2048 x
+        // 1024 5.7 / 6.5, 1000 x 2048 6.0 / 6.8, 3072 x 1024 7.7 / 6.6; 8 rows 512 x 256 6.2 / 11.3, 1000 x 1024 8.2 / 10.4, 1536 x
+        // 1024 12.4 / 10.9.
+        const int waves = (N + 8 * runtime_info().sm_count - 1) / (8 * runtime_info().sm_count);
+        if (TYPE == TYPE_Q8_0 && R < rows_per_pass && (long long)waves * (K + 200) <= (B == 1 ? 1300 : (B <= 4 ? 2450 : 2240))) ring_ok = false;
     }
     if (!ring_ok) {
         gemv_glu_simple_kernel<TYPE, B, dst_t><<<(N + 7) / 8, 256, 0, s>>>((const uint8_t*)wg, (const uint8_t*)wu, (const uint8_t*)vy, (dst_t*)dst, K,

@@ -81,6 +81,20 @@ def test_fused_glu_equals_plain_launches_and_epilogue(type_id, k, n, real, b):
     close(got, epilogue(g, u, "silu", dtype), dtype, scale=3.0 if dtype != torch.float32 else 64.0)
 
 
+# Both sides of the line between the plain and the ring kernel: stages of less than a pass, one wave of CTAs and the first row beyond.
+@pytest.mark.parametrize("type_id", [kq.Q8_0, kq.Q4_K])
+@pytest.mark.parametrize("k,n", [(256, 128), (256, 2369), (512, 1184), (512, 1185), (1024, 1184), (1024, 1185), (2048, 1000), (2048, 1185)])
+def test_fused_glu_on_small_matrices(type_id, k, n):
+    for b in (1, 2, 4, 5, 8):
+        for dtype in (torch.bfloat16, torch.float32):
+            wg, wu = (ops.upload_weights(random_packed(type_id, n, k, s), DT[type_id]) for s in (1, 2))
+            vy = ops.quantize_q8_1(seeded_acts(b, k, b, dtype).cuda())
+            got = ops.mmvq_fused_glu(DT[type_id], wg, wu, vy, n, k, b, dtype)
+            g, u = (ops.mmvq_plain(DT[type_id], w, vy, n, k, b, torch.float32) for w in (wg, wu))
+            close(got, epilogue(g, u, "silu", dtype), dtype, scale=3.0 if dtype != torch.float32 else 64.0)
+    assert_device_ok()
+
+
 @pytest.mark.parametrize("type_id", TYPES)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("activation", ["silu", "gelu", "relu", "gelu_erf", "sigmoid"])
