@@ -13,14 +13,14 @@
 //      multiplies 16 x 8 x 32 (Q6_K, whose scales cover 16 values: 16 x 8 x 16), and applies the scales to the sums where they are:
 //      in its registers. The W_k warps of a tile pair add up through shared memory in a fixed order (bit-reproducible).
 //
-// Bound by latency and issue slots of the unpacking and scaling before HBM (ncu, 28672 rows of Q4_K: 2.5 of 6.6 TB/s, an instruction
-// on 0.4 of the cycles). What keeps the instructions few: sums come out of the MMA as floats (the accumulator starts at the bits of
-// 1.5 * 2^23, so an exact subtraction takes the place of a conversion), scaling works on pairs of weight rows (fma.f32x2), a row's
-// block scales are decoded by one lane and passed on through shared memory. mma.sync and not tcgen05: scales differ from block to
+// Bound by latency and issue slots of the unpacking and scaling before HBM (ncu, an earlier form of the kernel, 28672 rows of Q4_K: 2.5
+// of 6.6 TB/s, an instruction on 0.4 of the cycles). What keeps the instructions few: sums come out of the MMA as floats (the
+// accumulator starts at the bits of 1.5 * 2^23, so an exact subtraction takes the place of a conversion), scaling works on pairs of
+// weight rows (fma.f32x2), a row's block scales are decoded by one lane and passed on through shared memory. mma.sync and not tcgen05: scales differ from block to
 // block, so a sum may not stay in the accumulator for more than 32 values; with tcgen05 every such sum goes out to TMEM and back, and
 // eight MMAs of 128 x 16 x 32 with their five barrier hand-offs per 256 k took 1400 cycles where HBM needs 420. Both launches,
-// matrices out of HBM, tcgen05 -> this: 4096 x 28672 Q4_K 4 rows 33.4 -> 24.9 us, 16 rows 46.9 -> 30.5; 14336 x 4096 Q6_K 16 rows
-// 53.5 -> 24.6; 4096 x 1024 Q4_K 16 rows 22.7 -> 6.9.
+// matrices out of HBM, tcgen05 -> this: 4096 x 28672 Q4_K 5 rows 36.6 -> 26.2 us, 16 rows 47.1 -> 32.9; 14336 x 4096 Q6_K 16 rows
+// 51.4 -> 25.7; 4096 x 1024 Q4_K 16 rows 22.1 -> 7.5.
 //
 // Every wait is bounded; a wait that gives up records a code in the device status word, and work is skipped.
 #include "common.cuh"
@@ -202,6 +202,11 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 // Sums of 32 / 16 products per output as the floats 1.5 * 2^23 + sum (|sum| < 2^22): activation rows g (lo) and g + 8 (hi), weight
 // rows 2t, 2t + 1. The weights are the MMA's N side: the factors of a pair of rows then come out of the record as the pair that
 // fma.f32x2 takes, where the other way round every factor has to be copied into both halves of a register pair.
@@ -253,11 +258,11 @@ template <int H, bool REF_ACTS> __device__ __forceinline__ void tcq_load_acts(co
     }
 }
 
-// acc[h] += the products of one 32-value block for weight rows 2t, 2t + 1 of eight and activation row 8 h + g: `w0 w1` the weights'
+// sum[h] = (b == 0) or += the products of one 32-value block for weight rows 2t, 2t + 1 of eight and activation row 8 h + g: `w0 w1` the weights'
 // fragment, `f` the rows' factors (Q4_K: d * sc pair, -dmin * m pair; Q6_K: the two halves' d * sc / 4 pairs; Q8_0: d pair, unused),
 // `b` the block of the pair held by `x`.
 template <int TYPE, int H>
-__device__ __forceinline__ void tcq_block(uint32_t w0, uint32_t w1, const TcqActs<H>& x, int b, const uint4& f, f32x2 (&acc)[H]) {
+__device__ __forceinline__ void tcq_block(uint32_t w0, uint32_t w1, const TcqActs<H>& x, int b, const uint4& f, f32x2 (&sum)[H]) {
     const f32x2 unbias = pack2(-12582912.0f, -12582912.0f), f0 = pack2(f.x, f.y), f1 = pack2(f.z, f.w);
     const uint32_t a[4] = {b ? x.q[0].z : x.q[0].x, H == 2 ? (b ? x.q[H - 1].z : x.q[H - 1].x) : 0u, b ? x.q[0].w : x.q[0].y,
                            H == 2 ? (b ? x.q[H - 1].w : x.q[H - 1].y) : 0u};
@@ -272,10 +277,14 @@ __device__ __forceinline__ void tcq_block(uint32_t w0, uint32_t w1, const TcqAct
     for (int h = 0; h < H; ++h) {
         const f32x2 xd = pack2(x.s[h][b].x, x.s[h][b].y), i = add2(d[h], unbias);
         if constexpr (TYPE == TYPE_Q6_K) {
-            acc[h] = fma2(xd, fma2(f0, i, mul2(f1, add2(e[h], unbias))), acc[h]);
+            const f32x2 t = fma2(f0, i, mul2(f1, add2(e[h], unbias)));
+            sum[h] = b == 0 ? mul2(xd, t) : fma2(xd, t, sum[h]);
+        } else if constexpr (TYPE == TYPE_Q8_0) {
+            const f32x2 f = mul2(f0, xd);  // exact: two f16 values
+            sum[h] = b == 0 ? mul2(f, i) : fma2(f, i, sum[h]);
         } else {
-            acc[h] = fma2(f0, mul2(xd, i), acc[h]);
-            if constexpr (TYPE == TYPE_Q4_K) acc[h] = fma2(f1, pack2(x.s[h][b].z, x.s[h][b].w), acc[h]);
+            const f32x2 xs = pack2(x.s[h][b].z, x.s[h][b].w);
+            sum[h] = fma2(f0, mul2(xd, i), b == 0 ? mul2(f1, xs) : fma2(f1, xs, sum[h]));
         }
     }
 }
@@ -323,9 +332,15 @@ template <bool ODD> __device__ __forceinline__ uint32_t tcq_word(uint32_t addr) 
 // One superblock of up to two tiles, i.e. `groups` = 4 or 2 groups of eight rows. Blocks come in pairs c (64 k); a pair's activations
 // serve all groups and the next pair's are loaded meanwhile (`cur` enters with pair 0 and leaves with pair 0 of superblock `next_sb`,
 // if that is not negative). box: shared address of row g's superblock; the next group's is 8 pitches on.
+//
+// Sums: a pair of blocks adds up by itself, the pairs of a superblock in `rest`, the superblocks in `acc`; what acc loses to rounding
+// stays in `rest` (compensated summation), and the warps' sums meet in double. One chain of f32 additions over a warp's blocks is the
+// faster one (28672 x 4096, 8 rows, us: Q4_K 25.2 against 26.5, Q6_K 39.2 / 39.5, Q8_0 36.6 / 40.0; 1024 x 4096 Q4_K 6.3 / 6.4) but
+// loses with its length. Relative error of f32 outputs against exact sums, chain / this, 3 rows of 14336 x 4096: Q8_0 1.5e-7 / 0.66e-7,
+// Q6_K 1.3e-7 / 0.71e-7, Q4_K 1.6e-7 / 0.86e-7 (the decode GEMV 0.76e-7, 0.77e-7, 1.45e-7; the tcgen05 form 1.1e-7, 1.1e-7, 1.6e-7).
 template <int TYPE, int H, bool REF_ACTS, bool ODD>
 __device__ __forceinline__ void tcq_superblock(const TcqParams& p, int sb, int next_sb, int lane, uint32_t box, uint32_t rec, int groups,
-                                               TcqActs<H>& cur, f32x2 (&acc)[4][H]) {
+                                               TcqActs<H>& cur, f32x2 (&acc)[4][H], f32x2 (&rest)[4][H]) {
     constexpr int PITCH = TcqType<TYPE>::PITCH;
     const int t = lane & 3;
     rec += t * TCQ_REC_PITCH;
@@ -368,6 +383,7 @@ __device__ __forceinline__ void tcq_superblock(const TcqParams& p, int sb, int n
                     a[1][i] = tcq_word<false>(row + 68 * c + 36 + 16 * i);
                 }
             }
+            f32x2 sum[H];
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 const uint32_t fa = rec + u * 4 * TCQ_REC_PITCH + 16 * (2 * c + b);
@@ -378,10 +394,22 @@ __device__ __forceinline__ void tcq_superblock(const TcqParams& p, int sb, int n
                 } else {
                     f = lds128(fa);
                 }
-                tcq_block<TYPE, H>(a[b][0], a[b][1], cur, b, f, acc[u]);
+                tcq_block<TYPE, H>(a[b][0], a[b][1], cur, b, f, sum);
             }
+#pragma unroll
+            for (int h = 0; h < H; ++h) rest[u][h] = add2(rest[u][h], sum[h]);
         }
         cur = nxt;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        if (u == 2 && groups < 4) break;
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            const f32x2 sum = add2(acc[u][h], rest[u][h]);
+            rest[u][h] = sub2(rest[u][h], sub2(sum, acc[u][h]));
+            acc[u][h] = sum;
+        }
     }
 }
 
@@ -444,9 +472,9 @@ __global__ void __launch_bounds__(32 * TcqType<TYPE>::WARPS, 1) gemv_rows_kernel
     bool ok = true;
     for (int pair = wm; pair < npairs; pair += wms) {
         const int tiles = min(2, ntiles - 2 * pair);
-        f32x2 acc[4][H];
+        f32x2 acc[4][H], rest[4][H];
 #pragma unroll
-        for (int i = 0; i < 4 * H; ++i) (&acc[0][0])[i] = 0ull;
+        for (int i = 0; i < 4 * H; ++i) (&acc[0][0])[i] = (&rest[0][0])[i] = 0ull;
         for (int sb = first_sb; sb < k1; sb += wks) {
             if (ok && !__all_sync(0xffffffffu, mbar_wait_bounded(&full[slot], ph))) {
                 if (lane == 0) record_failure(p.status, STATUS_WAIT_FULL_TIMEOUT, sb);
@@ -459,8 +487,8 @@ __global__ void __launch_bounds__(32 * TcqType<TYPE>::WARPS, 1) gemv_rows_kernel
                 __syncwarp();
                 const int next_sb = sb + wks < k1 ? sb + wks : (pair + wms < npairs ? first_sb : -1);
                 const uint32_t box = stage + (lane >> 2) * TT::PITCH;
-                if (TYPE == TYPE_Q6_K && (o & 2)) tcq_superblock<TYPE, H, REF_ACTS, true>(p, sb, next_sb, lane, box, exch, 2 * tiles, cur, acc);
-                else tcq_superblock<TYPE, H, REF_ACTS, false>(p, sb, next_sb, lane, box, exch, 2 * tiles, cur, acc);
+                if (TYPE == TYPE_Q6_K && (o & 2)) tcq_superblock<TYPE, H, REF_ACTS, true>(p, sb, next_sb, lane, box, exch, 2 * tiles, cur, acc, rest);
+                else tcq_superblock<TYPE, H, REF_ACTS, false>(p, sb, next_sb, lane, box, exch, 2 * tiles, cur, acc, rest);
                 ++used;
                 __syncwarp();  // every lane has read the stage and the record
                 issue();
@@ -477,7 +505,7 @@ __global__ void __launch_bounds__(32 * TcqType<TYPE>::WARPS, 1) gemv_rows_kernel
 #pragma unroll
             for (int h = 0; h < H; ++h) {
                 float v0, v1;
-                unpack2(acc[u][h], v0, v1);
+                unpack2(add2(acc[u][h], rest[u][h]), v0, v1);
                 sts64(exch + ((8 * h + (lane >> 2)) * TCQ_SUM_PITCH + 8 * u + 2 * (lane & 3)) * 4, __float_as_uint(v0), __float_as_uint(v1));
             }
         const auto group_sync = [&] {
@@ -490,8 +518,12 @@ __global__ void __launch_bounds__(32 * TcqType<TYPE>::WARPS, 1) gemv_rows_kernel
         dst_t* y = reinterpret_cast<dst_t*>(p.y) + grow;
         for (int tok = wk; tok < min(p.M, 8 * H); tok += wks) {
             const uint32_t src = exch0 + wm * wks * TCQ_EXCH_BYTES + (tok * TCQ_SUM_PITCH + lane) * 4;
-            float v = 0.0f;
-            for (int w = 0; w < wks; ++w) v += lds_f32(src + w * TCQ_EXCH_BYTES);
+            double part[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int w = 0; w < wks; w += 4)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    if (w + i < wks) part[i] += (double)lds_f32(src + (w + i) * TCQ_EXCH_BYTES);
+            const float v = (float)((part[0] + part[1]) + (part[2] + part[3]));
             if (row_ok) {
                 if (p.ksplit > 1) p.partial[((size_t)split * TCQ_TOKENS + tok) * p.N + grow] = v;
                 else y[(size_t)tok * p.ldy] = from_float<dst_t>(v);
@@ -505,9 +537,9 @@ __global__ void __launch_bounds__(32 * TcqType<TYPE>::WARPS, 1) gemv_rows_kernel
             if (*last_flag) {
                 __threadfence();
                 for (int tok = wk; tok < min(p.M, 8 * H); tok += wks) {
-                    float v = 0.0f;
-                    for (int s = 0; s < p.ksplit && row_ok; ++s) v += __ldcg(p.partial + ((size_t)s * TCQ_TOKENS + tok) * p.N + grow);
-                    if (row_ok) y[(size_t)tok * p.ldy] = from_float<dst_t>(v);
+                    double v = 0.0;
+                    for (int s = 0; s < p.ksplit && row_ok; ++s) v += (double)__ldcg(p.partial + ((size_t)s * TCQ_TOKENS + tok) * p.N + grow);
+                    if (row_ok) y[(size_t)tok * p.ldy] = from_float<dst_t>((float)v);
                 }
             }
         }

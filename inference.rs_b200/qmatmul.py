@@ -136,13 +136,13 @@ def prefers_mmvq(rows: int) -> bool:
 def _tier_overtakes(dtype: GgmlDType, rows: int, n: int, k: int) -> bool:
     """2..8 rows beyond that rule on which the tier's two launches cost less than the dp4a GEMV, if it takes the weights as they lie.
     The tier takes 6 us at least and hardly grows with the rows; the GEMV starts at 3.3 and grows with rows * n * k, the faster the
-    wider the rows are. GEMV / tier, us, weights out of HBM, on both sides of the lines: Q4_K k = 1024 3 rows 12288 7.45 / 7.70, 16384
-    8.56 / 8.19, 4 rows 8192 6.66 / 7.19, 12288 8.46 / 7.76; k = 2048 3 rows 4096 6.40 / 7.00, 8192 8.90 / 8.41; k = 4096 3 rows 1024
-    6.50 / 6.57, 2048 7.89 / 6.90. Q8_0 k = 1024 3 rows 12288 8.52 / 9.00, 16384 10.0 / 9.65; k = 4096 3 rows 1024 6.84 / 8.21, 2048
-    8.13 / 7.94; even counts cost its GEMV more, 4 rows k = 512 12288 6.15 / 6.95, k = 1024 4096 6.03 / 6.33, 6144 6.92 / 6.84. Q6_K k =
-    2048 3 rows 8192 9.80 / 10.9, 12288 13.0 / 12.9, 5 rows 1024 6.24 / 6.42, 4096 8.97 / 7.84; k = 4096 3 rows 2048 8.12 / 8.33, 4096
-    10.7 / 10.7. 2 rows, at any size: Q4_K 8.10 / 5.99 (512 x 256) to 79 / 48 (4096 x 65536), Q8_0 7.10 / 5.90 (256 x 256) to 171 / 77
-    (6144 x 65536), Q6_K 10.9 / 6.25 (2048 x 256) to 201 / 97; 6 rows of Q6_K 8.67 / 6.33 to 354 / 98."""
+    wider the rows are. GEMV / tier, us, weights out of HBM, on both sides of the lines: Q4_K k = 1024 3 rows 12288 7.47 / 7.66, 16384
+    8.56 / 8.19, 4 rows 8192 6.26 / 7.16, 12288 8.43 / 7.69; k = 2048 3 rows 4096 6.58 / 7.14, 8192 8.79 / 8.48; k = 4096 3 rows 1024
+    6.76 / 6.75, 2048 7.69 / 7.06. Q8_0 k = 1024 3 rows 12288 8.52 / 9.02, 16384 10.0 / 9.78; k = 4096 3 rows 1024 7.19 / 8.24, 2048
+    8.10 / 8.07; even counts cost its GEMV more, 4 rows k = 512 12288 5.82 / 7.03, k = 1024 4096 6.00 / 6.38, 6144 6.86 / 6.87, k = 1536
+    2048 6.60 / 6.17. Q6_K k = 2048 3 rows 8192 9.80 / 11.0, 12288 13.0 / 13.0, 5 rows 1024 6.67 / 6.42, 4096 8.98 / 8.12; k = 4096 3
+    rows 2048 8.12 / 8.29, 4096 10.6 / 10.9. 2 rows, at any size: Q4_K 8.28 / 6.16 (512 x 256) to 82 / 50 (4096 x 65536), Q8_0 6.66 / 5.85
+    (256 x 256) to 179 / 79 (6144 x 65536), Q6_K 10.8 / 6.25 (2048 x 256) to 203 / 99; 6 rows of Q6_K 7.99 / 6.41 to 358 / 100."""
     if not tensor_core_rows_supported(dtype, k):
         return False
     if rows == 2 or rows >= 6:

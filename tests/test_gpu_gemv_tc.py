@@ -17,6 +17,7 @@ from oracle import kquants as kq
 
 from oracle import refkernels as rk
 
+from inference_rs_b200 import QTensor
 from inference_rs_b200 import kernel_library as kl
 from inference_rs_b200 import ops
 from gpu_util import (DT, Q8_1_VS_CPU_PASS_FLOOR, TYPES, as_f32_numpy, assert_device_ok, elementwise_pass_rate, random_packed,
@@ -335,3 +336,48 @@ def test_blocks_of_nans_and_infinities_reach_the_outputs(type_id, m):
         pair = ops.mmvq_tc_plain(DT[type_id], w_dev, ops.mmvq_tc_quantize(x.cuda()), n, k, m, torch.float32)
         assert torch.equal(pair.isnan(), y.isnan())
     assert_device_ok()
+
+
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("n,k", [(64, 512), (2048, 2048), (4096, 14336), (28672, 4096)])
+def test_f32_outputs_lose_little_more_than_their_own_rounding(type_id, n, k):
+    """Relative error (2-norm) against exact sums of the same integer products and scales. An addition in f32 loses 2^-24 / sqrt(3) of
+    its result at most and about 0.7 of that over all mantissas; a chain of c terms loses sqrt(c / 2) times as much, so that pairs in
+    a chain of four, rounded products (two a block for Q6_K; for Q4_K also the min term, of twice the result's size), the rounding of
+    the output and nothing else give 0.6e-7 to 0.9e-7. A chain over the 64 to 128 blocks of a warp's rows gave 1.5e-7 to 2.2e-7."""
+    dt, k = DT[type_id], k_for(type_id, k)
+    gen = torch.Generator("cuda").manual_seed(n + k)
+    w = QTensor.quantize(torch.randn(n, k, device="cuda", generator=gen) * 0.02, dt)
+    dense = exact_values(type_id, w.packed_bytes(), n, k)
+    for m in (3, 12):
+        x = torch.randn(m, k, device="cuda", generator=gen)
+        blocks = ops.quantize_q8_1(x, k).view(m, k // 32, 36)
+        d = blocks[..., :2].contiguous().view(torch.float16).double()
+        ref = (d * blocks[..., 4:].contiguous().view(torch.int8).double()).view(m, k) @ dense.T
+        y = ops.gemv_tc(dt, w.data, x, n).double()
+        assert float((y - ref).norm() / ref.norm()) <= (1.0e-7 if type_id == kq.Q4_K else 0.8e-7)
+    assert_device_ok()
+
+
+def exact_values(type_id, packed, n, k):
+    """Dequantized weights in double: block scale times sub-scale times quant (minus the min) without a rounding."""
+    if type_id == kq.Q8_0:
+        b = packed.view(n, k // 32, 34)
+        return (b[..., :2].contiguous().view(torch.float16).double() * b[..., 2:].contiguous().view(torch.int8).double()).view(n, k)
+    if type_id == kq.Q6_K:
+        b = packed.view(n, k // 256, 210)
+        ql, qh = b[..., :128].view(n, -1, 2, 2, 32).int(), b[..., 128:192].view(n, -1, 2, 1, 32).int()
+        lo = torch.stack((ql[..., 0, :] & 15, ql[..., 1, :] & 15, ql[..., 0, :] >> 4, ql[..., 1, :] >> 4), dim=-2)
+        hi = torch.cat([(qh >> (2 * j)) & 3 for j in range(4)], dim=-2)
+        q = (lo | (hi << 4)) - 32  # [n, blocks, half, quarter, 32]
+        sc = b[..., 192:208].contiguous().view(torch.int8).view(n, -1, 16, 1).double()
+        d = b[..., 208:].contiguous().view(torch.float16).double().view(n, -1, 1, 1)
+        return (d * sc * q.reshape(n, -1, 16, 16).double()).view(n, k)
+    b = packed.view(n, k // 256, 144)
+    d, dmin = (b[..., 2 * i:2 * i + 2].contiguous().view(torch.float16).double() for i in (0, 1))
+    s = b[..., 4:16].int()
+    sc = torch.cat((s[..., :4] & 63, (s[..., 8:] & 15) | ((s[..., :4] >> 6) << 4)), -1)
+    mn = torch.cat((s[..., 4:8] & 63, (s[..., 8:] >> 4) | ((s[..., 4:8] >> 6) << 4)), -1)
+    q = b[..., 16:].view(n, -1, 4, 1, 32)
+    q = torch.cat((q & 15, q >> 4), dim=-2).reshape(n, -1, 8, 32).double()
+    return ((d * sc)[..., None] * q - (dmin * mn)[..., None]).view(n, k)
