@@ -229,7 +229,8 @@ const char* b200q_last_error(void);
 /* Options: "pdl" (launch GEMVs and quantizers with programmatic stream serialization), "force_simple_gemv",
  * "gemv_stage_bytes", "gemv_passes" (0 = the planner's choice, 1 or 2 passes of all warps per stage),
  * "gemv_pass_limit_bytes" (bytes one pass may cover before a row is given more warps), "gemv_ctas_per_sm", "tc_ksplit",
- * "gemm_direct", "gemv_one_kernel" (one-row GEMVs on the grouped kernel, default 1), "l2_prefetch_bytes" (see
+ * "gemm_direct", "gemm_pair_rows" (rows from which b200q_gemm_ws and b200q_mmq_ws use their workspace, -1 = their own
+ * rules), "gemv_one_kernel" (one-row GEMVs on the grouped kernel, default 1), "l2_prefetch_bytes" (see
  * b200q_set_weight_successor; 0 switches the prefetch off). get also answers "sm_count" and "smem_optin". Options are
  * process-wide tuning and test switches, read by every launch without synchronization: set them once, before the
  * threads that launch are started; the launchers themselves keep no other mutable state. */
@@ -325,7 +326,7 @@ long long b200q_mmq_workspace_bytes(int type, int M, int N, int K);
 int b200q_mmq_ws(int type, int elem, const void* w, const void* act_blocks, void* y, int M, int N, int K, int ldy, void* workspace,
                  long long workspace_bytes, void* stream);
 
-/* Small batches (M = 1..16 activation rows, B200Q_ERR_TOO_LARGE above) on the tcgen05 tensor cores with 8-bit integer
+/* Small batches (M = 1..16 activation rows, B200Q_ERR_TOO_LARGE above) on the tensor cores with 8-bit integer
  * operands: y[M][ldy] = x[M][ldx] . W[N][K]^T, x and y of element type `elem` (f32, f16 or bf16). Two launches on
  * `stream`: x is quantized into `workspace` (int8, one f16-rounded scale d = amax / 127 and the integer sum per 32
  * values: the layout kernel mmvq_tc_quantize of the reference, mmvq_gguf/mmvq_quantize.cu:157-190, computes the same

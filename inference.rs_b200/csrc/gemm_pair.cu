@@ -284,7 +284,8 @@ __device__ __forceinline__ uint2 lds_eight(uint32_t a) {
     return make_uint2(__funnelshift_r(lds32(w), b, sh), __funnelshift_r(b, lds32(w + 8), sh));
 }
 
-// HBM-bound. A thread takes eight packed bytes at a time and writes the 8 (Q8_0), 16 (Q4_K: low and high nibbles) or 32 (Q6_K: four
+// Between HBM and the issue slots, about half of either (ncu, 4096 x 14336 Q6_K: 29 us, 3.9 TB/s, an instruction on 0.5 of the cycles):
+// a CTA's loads, unpacking and stores follow one another. A thread takes eight packed bytes at a time and writes the 8 (Q8_0), 16 (Q4_K: low and high nibbles) or 32 (Q6_K: four
 // quarters) values they hold a part of, in 16-byte stores; neighbouring threads write neighbouring pieces. The 34- and 210-byte blocks
 // of Q8_0 and Q6_K are aligned to 2 bytes only: a CTA first brings its values' packed bytes into shared memory by 16-byte loads
 // (expansion and product, against reading them by halves: 512 x 4096 x 14336 Q8_0 85.1 -> 81.4 us, 333 x 6144 x 4096 34.3 -> 32.9,
@@ -489,11 +490,13 @@ static bool gemm_pair_pays(int type, int M, int N, int K) {
     return 24 * tiles < twenty_fourths * sms;
 }
 size_t gemm_pair_workspace_bytes(int type, int M, int N, int K) { return gemm_pair_pays(type, M, N, K) ? (size_t)N * K * 2 : 0; }
-// quantized activations: their 16-bit copy as well. The single-launch kernel expands them in every tile, so this pays wherever that
-// kernel serves the launcher; the shapes it does not take are multiplied as integers by its plain kernel, and stay so.
+// Quantized activations: their 16-bit copy as well. The single-launch kernel expands them in every tile, so this pays at every row count
+// on every shape that kernel serves, us launcher / this, Q4_K: 28672 x 4096 17 rows 105 / 99, 128 rows 125 / 100, 256 152 / 108; 14336 x
+// 4096 17 rows 58 / 47, 128 63 / 49; 1024 x 1024 17 rows 19.5 / 11.5 (closest: Q8_0 28672 x 4096 at 17 rows, 109 / 108). The shapes it does
+// not take are multiplied as integers by its plain kernel, and stay so.
 size_t mmq_pair_workspace_bytes(int type, int M, int N, int K) {
     const bool tiles = K % 256 == 0 && (long long)K / type_block_elems(type) * type_block_bytes(type) % 16 == 0;
-    return tiles ? ((size_t)N * K + (size_t)M * K) * 2 : 0;
+    return tiles && M >= runtime_info().gemm_pair_rows ? ((size_t)N * K + (size_t)M * K) * 2 : 0;
 }
 
 // The reference launchers' product (launch_mmq_gguf_*, gemm_tcgen05.cu) with a workspace: bf16 operands, f32 accumulation.

@@ -21,8 +21,8 @@ struct RuntimeInfo {
     int force_simple;      // route every GEMV to the simple kernel (testing)
     int gemv_stage_target; // bytes per shared-memory stage the GEMV planner aims at
     int gemm_direct;       // 1: the GEMM reads packed weights straight from global memory (no shared-memory staging)
-    int gemm_pair_rows;    // GEMM with a workspace: rows from which the weights are expanded and CTA pairs used (-1: the rule of
-                           // gemm_pair.cu)
+    int gemm_pair_rows;    // GEMM and prefill product with a workspace: rows from which the weights are expanded and CTA pairs used
+                           // (-1: the rules of gemm_pair.cu)
     int gemv_ctas_per_sm;  // CTAs of one GEMV grid per SM: 2, or 1 to leave the other slot to the next grid
     int tc_ksplit;         // small-batch tensor-core kernel: split K over CTAs for matrices with few rows (1, testing: 0)
     int gemv_one_kernel;   // one-row GEMVs on raw activations run on the grouped kernel, so that a decode chain alternates

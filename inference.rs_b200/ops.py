@@ -212,8 +212,10 @@ def _device_numbers(device: torch.device) -> tuple[int, int]:
 
 
 def mmq(dtype: GgmlDType, w: torch.Tensor, vy: torch.Tensor, m: int, n: int, k: int, out_dtype: torch.dtype) -> torch.Tensor:
-    """`launch_mmq_gguf_<type>` on activation blocks `vy` from `quantize_mmq_q8_1(x, MMQ_LAYOUT[dtype])`; returns
-    [m, n] of `out_dtype`, called as the reference's host calls it (crates/inference-quant/src/gguf/fast_mmq.rs:489-512)."""
+    """The product of `launch_mmq_gguf_<type>` on activation blocks `vy` from `quantize_mmq_q8_1(x, MMQ_LAYOUT[dtype])`; returns
+    [m, n] of `out_dtype`. `b200q_mmq_ws` with 2 (n + m) k bytes from torch's allocator where it takes the shape and the memory is
+    there (same bits, half the time), else that launcher, called as the reference's host calls it
+    (crates/inference-quant/src/gguf/fast_mmq.rs:489-512)."""
     cc, nsm = _device_numbers(w.device) if w.is_cuda else (0, 0)  # (off the GPU: the check below raises)
     dst = kl.host().mmq(dtype, w, vy, m, n, k, elem_of(out_dtype), cc, nsm)
     if dst is not None:

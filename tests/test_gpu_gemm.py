@@ -22,7 +22,10 @@ from oracle import kquants as kq
 
 from oracle import refkernels as rk
 
+from inference_rs_b200 import kernel_library as kl
 from inference_rs_b200 import ops
+from inference_rs_b200.dtypes import MMQ_TYPE_X
+from inference_rs_b200.ops import elem_of
 from gpu_util import DT, TYPES, as_f32_numpy, assert_device_ok, random_packed, real_packed, seeded_acts, seeded_weights
 
 pytestmark = pytest.mark.gpu
@@ -32,6 +35,23 @@ def rounded_weights(type_id, packed, k, dtype):
     w = kq.dequantize(type_id, packed, k)
     t = torch.from_numpy(w).to(dtype).float().numpy()
     return t.astype(np.float64)
+
+
+def single_launch(dt, w, x, n):
+    """`b200q_gemm`: every weight tile expanded inside the kernel that multiplies it, no workspace."""
+    (m, k), y = x.shape, torch.empty(x.shape[0], n, dtype=x.dtype, device="cuda")
+    kl.check(kl.library().b200q_gemm(int(dt), elem_of(x.dtype), w.data_ptr(), x.data_ptr(), y.data_ptr(), m, n, k, k, n,
+                                     torch.cuda.current_stream().cuda_stream), "b200q_gemm")
+    return y
+
+
+def mmq_launcher(dt, w, vy, m, n, k, dtype):
+    """`launch_mmq_gguf_<type>` itself, as a host that links the symbol calls it (fast_mmq.rs:489-512); `ops.mmq` lends a workspace."""
+    y = torch.empty(m, n, dtype=dtype, device="cuda")
+    getattr(kl.library(), f"launch_mmq_gguf_{dt.tag}")(None, w.data_ptr(), vy.data_ptr(), y.data_ptr(), k, n, m, k // dt.block_size, n, 1000, 148, 232448,
+                                                       32, MMQ_TYPE_X[elem_of(dtype)], torch.cuda.current_stream().cuda_stream)
+    assert kl.library().b200q_take_launch_status() == 0
+    return y
 
 
 def run_gemm(type_id, m, n, k, dtype=torch.bfloat16, packed=None, seed=0, check_cpu=True, real=None, sample_rows=None):
@@ -45,6 +65,8 @@ def run_gemm(type_id, m, n, k, dtype=torch.bfloat16, packed=None, seed=0, check_
     y = ops.gemm(DT[type_id], w_dev, x_dev, n)
     torch.cuda.synchronize()
     assert_device_ok()
+    # whichever form that took: the single launch gives the same bits
+    assert torch.equal(y, single_launch(DT[type_id], w_dev, x_dev, n))
     rows = np.arange(m)
     if sample_rows is not None and sample_rows < m:
         rows = np.sort(np.random.default_rng(seed).choice(m, size=sample_rows, replace=False))
@@ -91,7 +113,7 @@ def test_prefill_shapes_m512(type_id, k, n):
 @pytest.mark.parametrize("k,n", [(4096, 4096), (14336, 4096)])
 @pytest.mark.parametrize("m", [2048, 8192])
 def test_prefill_shapes_large_m(type_id, k, n, m):
-    # M = 2048 with enough tiles takes the 256-token CTA tile; M = 8192 is the compute-bound end of the sweep
+    # the single launch takes its 256-token CTA tile at M = 2048 where there are enough tiles; M = 8192 is the compute-bound end of the sweep
     run_gemm(type_id, m, n, k, packed=real_packed(type_id, n, k), seed=m, real=True, sample_rows=192)
 
 
@@ -113,7 +135,6 @@ def test_rows_are_independent():
 
 
 def test_unsupported_inputs_are_refused():
-    from inference_rs_b200 import kernel_library as kl
     w_dev = ops.upload_weights(random_packed(kq.Q4_K, 128, 256, 1), DT[kq.Q4_K])
     with pytest.raises(TypeError):
         ops.gemm(DT[kq.Q4_K], w_dev, torch.zeros(32, 256, device="cuda", dtype=torch.float64), 128)
@@ -149,9 +170,11 @@ def run_mmq(type_id, m, n, k, dtype=torch.bfloat16, packed=None, seed=0, real=No
     w_dev = ops.upload_weights(packed, DT[type_id])
     layout = ops.MMQ_LAYOUT[DT[type_id]]
     vy = ops.quantize_mmq_q8_1(x.cuda(), layout)
-    y = ops.mmq(DT[type_id], w_dev, vy, m, n, k, dtype)
+    y = mmq_launcher(DT[type_id], w_dev, vy, m, n, k, dtype)
     torch.cuda.synchronize()
     assert_device_ok()
+    # the form with a workspace: bf16 products in the same order (shapes it does not take go to the launcher)
+    assert torch.equal(ops.mmq(DT[type_id], w_dev, vy, m, n, k, dtype), y)
     rows = np.arange(m)
     if sample_rows is not None and sample_rows < m:
         rows = np.sort(np.random.default_rng(seed).choice(m, size=sample_rows, replace=False))
@@ -253,3 +276,12 @@ def test_expansion_of_ragged_pieces_and_even_addresses(type_id, n, k, off):
     torch.cuda.synchronize()
     assert_device_ok()
     assert torch.equal(pair, single)
+
+
+# The launcher's own tile kernel on quantized activations: one and two 128-token sub-tiles per CTA, ragged in both directions.
+@pytest.mark.parametrize("type_id", TYPES)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("m,n", [(1, 64), (129, 18945), (255, 19000)])
+def test_mmq_launcher_token_tiles_and_output_types(type_id, dtype, m, n):
+    k = 512 if type_id != kq.Q6_K else 2048
+    run_mmq(type_id, m, n, k, dtype=dtype, packed=random_packed(type_id, n, k, seed=m), seed=m, real=False, sample_rows=48)
