@@ -13,8 +13,8 @@
 //      multiplies 16 x 8 x 32 (Q6_K, whose scales cover 16 values: 16 x 8 x 16), and applies the scales to the sums where they are:
 //      in its registers. The W_k warps of a tile pair add up through shared memory in a fixed order (bit-reproducible).
 //
-// Bound by latency and issue slots of the unpacking and scaling before HBM (ncu, an earlier form of the kernel, 28672 rows of Q4_K: 2.5
-// of 6.6 TB/s, an instruction on 0.4 of the cycles). What keeps the instructions few: sums come out of the MMA as floats (the
+// Bound by latency and issue slots of the unpacking and scaling before HBM (ncu, 28672 rows of Q4_K, 8 activation
+// rows: 2.3 of 6.6 TB/s, an instruction on 0.36 of the cycles). What keeps the instructions few: sums come out of the MMA as floats (the
 // accumulator starts at the bits of 1.5 * 2^23, so an exact subtraction takes the place of a conversion), scaling works on pairs of
 // weight rows (fma.f32x2), a row's block scales are decoded by one lane and passed on through shared memory. mma.sync and not tcgen05: scales differ from block to
 // block, so a sum may not stay in the accumulator for more than 32 values; with tcgen05 every such sum goes out to TMEM and back, and

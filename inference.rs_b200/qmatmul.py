@@ -17,9 +17,8 @@ from . import kernel_library as kl
 MMVQ_MAX_BATCH = 8  # rows the decode GEMV launchers take (fast_mmvq.rs:84)
 TENSOR_CORE_MAX_ROWS = 16  # rows the small-batch tensor-core kernel takes (fast_mmvq.rs:86)
 
-# 3..8 rows: the crossovers measured on B200 against the dp4a GEMV at the Llama-3-8B shapes. The tier's cost hardly
-# grows with the row count, the GEMV's grows linearly; Q6_K's unpacking is the most expensive, so it needs more rows
-# or a bigger matrix. 9..16 rows: always (the alternative is the prefill GEMM).
+# 3..8 rows that always took the tier, at any address: weights off the 16-byte boundaries it needs are refused there, as ever.
+# `_tier_overtakes` adds the rows on which it is the faster one as well.
 
 
 def _tensor_core_pays(dtype: GgmlDType, rows: int, n: int, k: int) -> bool:
@@ -35,8 +34,8 @@ def tensor_core_rows_supported(dtype: GgmlDType, k: int) -> bool:
 
 
 def prefers_tensor_core_rows(dtype: GgmlDType, rows: int, n: int, k: int) -> bool:
-    """The small-batch tensor-core tier (fast_mmvq.rs:118-134: 2..16 rows where a type has it). Here: 9..16 rows
-    always, 3..8 rows from the measured crossover with the dp4a GEMV on; 1..2 rows stay on the one-launch GEMV."""
+    """The small-batch tensor-core tier without a way back (fast_mmvq.rs:118-134: 2..16 rows where a type has it). Here: 9..16 rows
+    always (the alternative is the prefill GEMM), 3..8 rows on big matrices or from 5 (Q6_K 7) rows on; `_tier` decides for all."""
     if rows > TENSOR_CORE_MAX_ROWS or rows < 3 or not tensor_core_rows_supported(dtype, k):
         return False
     return rows > MMVQ_MAX_BATCH or _tensor_core_pays(dtype, rows, n, k)

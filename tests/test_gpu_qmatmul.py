@@ -88,7 +88,7 @@ def test_rows_3_to_16_take_the_tensor_core_tier_where_it_pays(type_id):
             cpu = kq.matmul(type_id, as_f32_numpy(x), packed, n)
             err = np.abs(as_f32_numpy(y) - cpu).max()
             assert err <= 1e-3 + 1e-2 * np.abs(cpu).max(), (rows, dtype, err)
-    # the tier's scratch keeps its address per stream, so a captured forward can be replayed
+    # under capture the tier's scratch comes from the graph's own memory pool, so a captured forward can be replayed
     x = seeded_acts(12, k, 90, torch.bfloat16).cuda()
     eager = qmm.forward(x)
     stream = torch.cuda.Stream()

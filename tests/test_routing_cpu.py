@@ -11,7 +11,7 @@ LLAMA_SHAPES = [(4096, 6144), (4096, 4096), (4096, 28672), (14336, 4096), (4096,
 
 
 @pytest.mark.parametrize("dtype", [GgmlDType.Q4K, GgmlDType.Q6K, GgmlDType.Q8_0])
-def test_rows_1_2_stay_on_the_gemv_and_9_to_16_take_the_tensor_core_tier(dtype):
+def test_rows_9_to_16_take_the_tensor_core_tier_and_1_2_never_without_a_way_back(dtype):
     for k, n in LLAMA_SHAPES:
         for rows in (1, 2):
             assert not qm.prefers_tensor_core_rows(dtype, rows, n, k) and qm.prefers_mmvq(rows)
@@ -20,7 +20,7 @@ def test_rows_1_2_stay_on_the_gemv_and_9_to_16_take_the_tensor_core_tier(dtype):
         assert not qm.prefers_tensor_core_rows(dtype, 17, n, k) and not qm.prefers_mmvq(17)
 
 
-def test_rows_3_to_8_follow_the_measured_crossovers():
+def test_rows_3_to_8_that_take_the_tier_without_a_way_back():
     # light unpacking (Q4_K, Q8_0): from 5 rows everywhere, from 3 rows on big matrices
     for dtype in (GgmlDType.Q4K, GgmlDType.Q8_0):
         assert not qm.prefers_tensor_core_rows(dtype, 4, 4096, 4096)
