@@ -920,7 +920,7 @@ def main():
                     xb = torch.randn(b, k, device="cuda", generator=gen).to(torch.bfloat16)
                     qms[0].forward(xb)
                     us = time_launch_list(torch, stream, [(lambda q=q: q.forward(xb)) for q in qms], max(3, int(2e9 // (wbytes * copies))))
-                    kern = ("gemv_tc" if _qm.prefers_tensor_core_rows(dt, b, n, k) else ("gemv" if b <= 8 else "gemm"))
+                    kern = ("gemv", "gemv_tc", "gemm", "gemv_tc")[_qm._tier(dt, b, n, k, ops.ACT_QUANT_Q8_1)]
                     small.append({"type": dt.name, "k": k, "n": n, "b": b, "kernel": kern, "us": round(us, 2),
                                   "GBps": round((wbytes + b * k * 2 + b * n * 2) / us / 1e3, 1),
                                   "frac_of_measured_hbm": round((wbytes + b * k * 2 + b * n * 2) / us / 1e3 / peak, 3)})
